@@ -1,7 +1,8 @@
-// FP64 ground-state kernels: Gram-Schmidt, the band-by-band CG of the
-// reference, and the pieces of the subspace diagonalisation (H_sub = U^H H U,
-// Hermitian eigen-decomposition, rotation).  Every reduction is a fixed-order
-// CTA reduction (deterministic).  Arrays: zu_GS(NL,NB,NK_s:NK_e) complex(8).
+// FP64 ground-state kernels: the one-by-one Gram-Schmidt, the band-by-band CG of
+// the reference, and the Hermitian eigen-decomposition of the subspace
+// diagonalisation (its products and the blocked Gram-Schmidt are in k_zgemm.cu).
+// Every reduction is a fixed-order sum (deterministic).  Arrays:
+// zu_GS(NL,NB,NK_s:NK_e) complex(8).
 #include <cuda_runtime.h>
 
 #include <cooperative_groups.h>
@@ -15,23 +16,32 @@ namespace sgpu {
 constexpr int GS_THREADS = 512;
 
 // ------------------------------------------------------------------ groups --
-// The Gram-Schmidt and CG kernels run one thread-block cluster per k-point: the
-// cluster's C CTAs split the NL points into contiguous slices, and every inner
-// product is a fixed-order CTA sum followed by a sum of the C partials in rank
-// order, read from each CTA's shared memory over the cluster (distributed
-// shared memory); all CTAs of the cluster obtain the same value.  The
-// sequential structure of the reference (band by band, each projection on the
-// already updated vector) is kept; the cluster only parallelises each vector
-// operation over more SMs.  C = 1 is one CTA per k-point.
+// The CG and one-by-one Gram-Schmidt kernels run one thread-block cluster per
+// k-point: the cluster's C CTAs split the NL points into contiguous slices, and
+// every inner product is a fixed-order CTA sum followed by a sum of the C partials
+// in rank order, read from each CTA's shared memory over the cluster (distributed
+// shared memory); all CTAs of the cluster obtain the same value.  C = 1 is one CTA
+// per k-point.
 namespace cgx = cooperative_groups;
+
+constexpr int GRP_NV = 8;    // values of one sum
+constexpr int CGB = 256;     // lower bands projected out together (grp_project)
+
+struct GrpShared {
+  double sh[32 * GRP_NV];
+  double part[2][GRP_NV];    // this CTA's partial sums (double-buffered)
+  double tot[GRP_NV];
+  double2 dots[2][CGB];      // this CTA's inner products with the lower bands (double-buffered)
+  double2 d[CGB], c[CGB];
+};
 
 struct Grp {
   int k, rank, C, lo, hi;
-  int parity;
-  double* part;  // [2][4] this CTA's partial sums (shared memory)
+  int parity, dparity;
+  GrpShared* s;
 };
 
-__device__ __forceinline__ Grp grp_make(int NL, double* part) {
+__device__ __forceinline__ Grp grp_make(int NL, GrpShared* s) {
   cgx::cluster_group cl = cgx::this_cluster();
   Grp g;
   g.C = (int)cl.num_blocks();
@@ -41,30 +51,30 @@ __device__ __forceinline__ Grp grp_make(int NL, double* part) {
   g.lo = min(NL, g.rank * slice);
   g.hi = min(NL, g.lo + slice);
   g.parity = 0;
-  g.part = part;
+  g.dparity = 0;
+  g.s = s;
   return g;
 }
 
 // sum of NV doubles over the k-point's cluster, valid in every thread of every CTA
 template <int NV>
-__device__ __forceinline__ void grp_allsum(Grp& g, double (&v)[NV], double* sh) {
-  block_allsum<NV>(v, sh);
+__device__ __forceinline__ void grp_allsum(Grp& g, double (&v)[NV]) {
+  static_assert(NV <= GRP_NV, "the exchange holds GRP_NV values");
+  block_allsum<NV>(v, g.s->sh);
   if (g.C == 1) return;
   cgx::cluster_group cl = cgx::this_cluster();
   if (threadIdx.x == 0)
 #pragma unroll
-    for (int j = 0; j < NV; ++j) g.part[g.parity * 4 + j] = v[j];
+    for (int j = 0; j < NV; ++j) g.s->part[g.parity][j] = v[j];
   cl.sync();  // every CTA's partial is in place (and every read of this slot from two sums ago is done)
-  double t[NV];
-#pragma unroll
-  for (int j = 0; j < NV; ++j) t[j] = 0.0;
-  for (int r = 0; r < g.C; ++r) {
-    const double* rp = cl.map_shared_rank(g.part, r);
-#pragma unroll
-    for (int j = 0; j < NV; ++j) t[j] += rp[g.parity * 4 + j];
+  if (threadIdx.x < NV) {
+    double t = 0.0;
+    for (int r = 0; r < g.C; ++r) t += cl.map_shared_rank(&g.s->part[g.parity][0], r)[threadIdx.x];
+    g.s->tot[threadIdx.x] = t;
   }
+  __syncthreads();
 #pragma unroll
-  for (int j = 0; j < NV; ++j) v[j] = t[j];
+  for (int j = 0; j < NV; ++j) v[j] = g.s->tot[j];
   g.parity ^= 1;
 }
 
@@ -73,50 +83,50 @@ __device__ __forceinline__ void grp_exit(const Grp& g) {
   if (g.C > 1) cgx::this_cluster().sync();
 }
 
+// acc += (Re, Im) conj(a) b
+__device__ __forceinline__ void zdot_add(double& re, double& im, double2 a, double2 b) {
+  re = fma(a.x, b.x, fma(a.y, b.y, re));
+  im = fma(a.x, b.y, fma(-a.y, b.x, im));
+}
+__device__ __forceinline__ double rdot(double2 a, double2 b, double acc) { return fma(a.x, b.x, fma(a.y, b.y, acc)); }
+
 // <a|b> over the NL points (the cluster's sum), valid in every thread
-__device__ __forceinline__ double2 grp_zdot(Grp& g, const double2* __restrict__ a, const double2* __restrict__ b,
-                                            double* sh) {
+__device__ __forceinline__ double2 grp_zdot(Grp& g, const double2* __restrict__ a, const double2* __restrict__ b) {
   double v[2] = {0.0, 0.0};
-  for (int i = g.lo + threadIdx.x; i < g.hi; i += blockDim.x) {
-    const double2 x = a[i], y = b[i];
-    v[0] = fma(x.x, y.x, fma(x.y, y.y, v[0]));
-    v[1] = fma(x.x, y.y, fma(-x.y, y.x, v[1]));
-  }
-  grp_allsum<2>(g, v, sh);
+  for (int i = g.lo + threadIdx.x; i < g.hi; i += blockDim.x) zdot_add(v[0], v[1], a[i], b[i]);
+  grp_allsum<2>(g, v);
   return make_double2(v[0], v[1]);
 }
 
-__device__ __forceinline__ double grp_nrm2(Grp& g, const double2* __restrict__ a, double* sh) {
+__device__ __forceinline__ double grp_nrm2(Grp& g, const double2* __restrict__ a) {
   double v[1] = {0.0};
-  for (int i = g.lo + threadIdx.x; i < g.hi; i += blockDim.x) {
-    const double2 x = a[i];
-    v[0] = fma(x.x, x.x, fma(x.y, x.y, v[0]));
-  }
-  grp_allsum<1>(g, v, sh);
+  for (int i = g.lo + threadIdx.x; i < g.hi; i += blockDim.x) v[0] = rdot(a[i], a[i], v[0]);
+  grp_allsum<1>(g, v);
   return v[0];
 }
 
 #define GRP_FOR(i) for (int i = g.lo + threadIdx.x; i < g.hi; i += blockDim.x)
 
 // ------------------------------------------------------------ Gram-Schmidt --
-// Gram_Schmidt_ompk (GS/Gram_Schmidt.f90:32-55): for each band, subtract the
-// projections on the lower bands one by one (each projection uses the band as
-// already updated), then normalise.  One cluster per k-point.
-__global__ void __launch_bounds__(GS_THREADS) k_gram_schmidt(double2* __restrict__ zu, int NB, int NL, double Hxyz) {
-  __shared__ double sh[64];
-  __shared__ double part[8];
-  Grp g = grp_make(NL, part);
-  double2* base = zu + (size_t)g.k * NB * NL;
-  for (int ib = 0; ib < NB; ++ib) {
+// Gram_Schmidt_ompk (GS/Gram_Schmidt.f90:32-55) as the reference does it, for the
+// bands p0 .. p0+pb-1 of the k-points the blocked form refuses (bad[k], see
+// k_zgemm.cu; the bands below p0 are already projected out): for each band, subtract
+// the projections on the panel's lower bands one by one, then normalise.
+__global__ void __launch_bounds__(GS_THREADS) k_gram_schmidt(double2* __restrict__ zu, int NB, int NL, double Hxyz,
+                                                            int p0, int pb, const int* __restrict__ bad) {
+  __shared__ GrpShared sm;
+  Grp g = grp_make(NL, &sm);
+  if (!bad[g.k]) return;  // the whole cluster
+  double2* base = zu + ((size_t)g.k * NB + p0) * NL;
+  for (int ib = 0; ib < pb; ++ib) {
     double2* u = base + (size_t)ib * NL;
     for (int ibt = 0; ibt < ib; ++ibt) {
       const double2* ut = base + (size_t)ibt * NL;
-      const double2 d = grp_zdot(g, ut, u, sh);
+      const double2 d = grp_zdot(g, ut, u);
       const double2 zov = make_double2(d.x * Hxyz, d.y * Hxyz);
       GRP_FOR(i) u[i] = csub(u[i], cmul(ut[i], zov));
     }
-    const double s = grp_nrm2(g, u, sh) * Hxyz;
-    const double inv = 1.0 / sqrt(s);
+    const double inv = 1.0 / sqrt(grp_nrm2(g, u) * Hxyz);
     GRP_FOR(i) u[i] = make_double2(u[i].x * inv, u[i].y * inv);
   }
   grp_exit(g);
@@ -125,10 +135,26 @@ __global__ void __launch_bounds__(GS_THREADS) k_gram_schmidt(double2* __restrict
 // ---------------------------------------------------------------------- CG --
 // CG_ompk with skip_gsortho='n' (GS/CG.f90:34-139), split into kernels around
 // the H applications; one cluster per k-point works on band ib of its k-point.
-// Work vectors W[which][k][NL] (which = xk, hxk, txk, gk, pk, pko, htpsi, ttpsi):
-// each kind is a contiguous batch of one vector per k-point for the H pass.
-// Every CTA reads the k-point's state at the start of a kernel; rank 0 writes it
-// back only after a cluster-wide sum, i.e. after every CTA has read it.
+// Work vectors W[which][k][NL]: each kind is a contiguous batch of one vector per
+// k-point for the H application.  Every CTA reads the k-point's state at the start
+// of a kernel; rank 0 writes it back only after a cluster-wide sum, i.e. after every
+// CTA has read it.
+//
+// Projections on the lower bands.  The reference subtracts them one by one, each
+// inner product taken with the vector as already updated: ib dependent sums.  In
+// terms of the inner products with the original vector, d_j = <u_j|x>, those
+// coefficients solve the unit triangular system
+//     c_j = d_j - sum_{i<j} <u_j|u_i> c_i,    c = (I + L)^-1 d,
+// (modified Gram-Schmidt in its inverse compact WY form: Swirydowicz, Langou,
+// Ananthan, Yang and Thomas, Numer. Linear Algebra Appl. 28 (2021) e2343), so one
+// exchange gives all of them and the result is the reference's up to rounding, also
+// where the bands are not orthogonal to each other (they are not: the reference
+// orthogonalises a new band with the real parts of its overlaps, CG.f90:45,70).
+// (I + L)^-1 grows by one row per finished band: gs_M, and gs_MR for the real parts.
+// Lower bands are taken in blocks of CGB, block after block, so one row holds the
+// CGB columns of its own block.
+// At 32^3, two k-points, 144 bands, TPA, 4 iterations: sgpu_cg + 2 Gram-Schmidt 808
+// ms with dependent sums; the measured time now stands at launch_cg_project.
 enum { CG_XK = 0, CG_HXK, CG_TXK, CG_GK, CG_PK, CG_PKO, CG_HT, CG_TT, CG_HK, CG_NW };
 
 struct CGState {
@@ -140,225 +166,426 @@ __device__ __forceinline__ double2* wv(double2* W, int nkl, int k, int which, in
   return W + ((size_t)which * nkl + k) * NL;
 }
 
-// Orthogonalise band ib against the lower bands with REAL coefficients (s is
-// real(8) in the reference, CG.f90:45,70), normalise into xk.
-__global__ void __launch_bounds__(GS_THREADS) k_cg_begin(double2* __restrict__ zu, double2* __restrict__ W,
-                                                         CGState* __restrict__ st, int ib, int nkl, int NB, int NL,
-                                                         double Hxyz) {
-  __shared__ double sh[64];
-  __shared__ double part[8];
-  Grp g = grp_make(NL, part);
-  const int k = g.k;
-  double2* base = zu + (size_t)k * NB * NL;
-  double2* u = base + (size_t)ib * NL;
-  for (int ibt = 0; ibt < ib; ++ibt) {
-    const double2* ut = base + (size_t)ibt * NL;
-    const double s = grp_zdot(g, ut, u, sh).x * Hxyz;
-    GRP_FOR(i) u[i] = make_double2(u[i].x - ut[i].x * s, u[i].y - ut[i].y * s);
-  }
-  const double inv = 1.0 / sqrt(grp_nrm2(g, u, sh) * Hxyz);
-  double2* xk = wv(W, nkl, k, CG_XK, NL);
-  GRP_FOR(i) xk[i] = make_double2(u[i].x * inv, u[i].y * inv);
-  if (g.rank == 0 && threadIdx.x == 0) { st[k].done = 0; st[k].iters = 0; }
-  grp_exit(g);
+// everything the CG kernels of one handle share
+struct CGArgs {
+  double2* zu;       // [nkl][NB][NL]
+  double2* W;        // [CG_NW][nkl][NL]
+  CGState* st;       // [nkl]
+  double2* M;        // [nkl][NB][CGB] rows of (I + L)^-1
+  double* MR;        // [nkl][NB][CGB] the same for the real parts of the overlaps
+  double* tband;     // [nkl] kinetic energy of xk
+  int nkl, NB, NL;
+  double Hxyz;
+};
+
+__device__ __forceinline__ double warp_sum_gs(double v) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
 }
 
-// xkHxk = Re <xk|hxk> Hxyz
-__global__ void __launch_bounds__(GS_THREADS) k_cg_dot0(double2* __restrict__ W, CGState* __restrict__ st, int nkl,
-                                                        int NL, double Hxyz) {
-  __shared__ double sh[64];
-  __shared__ double part[8];
-  Grp g = grp_make(NL, part);
-  const int k = g.k;
-  const double d = grp_zdot(g, wv(W, nkl, k, CG_XK, NL), wv(W, nkl, k, CG_HXK, NL), sh).x * Hxyz;
-  if (g.rank == 0 && threadIdx.x == 0) st[k].xkHxk = d;
-  grp_exit(g);
+// c = (I + L)^-1 d for the n bands of one block, one warp per row.  row: row 0 of the
+// block in gs_M / gs_MR.
+template <bool REAL>
+__device__ __forceinline__ void cg_solve(const double2* __restrict__ M, const double* __restrict__ MR, int n,
+                                         const double2* d, double2* c) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int j = warp; j < n; j += nw) {
+    double2 v = make_double2(0.0, 0.0);
+    if (REAL) {
+      for (int i = lane; i <= j; i += 32) v.x = fma(MR[(size_t)j * CGB + i], d[i].x, v.x);
+      v.x = warp_sum_gs(v.x);
+    } else {
+      for (int i = lane; i <= j; i += 32) v = cfma(M[(size_t)j * CGB + i], d[i], v);
+      v.x = warp_sum_gs(v.x);
+      v.y = warp_sum_gs(v.y);
+    }
+    if (lane == 0) c[j] = v;
+  }
 }
 
-// gradient, orthogonalisation against the lower bands, conjugate direction,
-// pko = normalised component of pk orthogonal to xk (CG.f90:85-106)
-__global__ void __launch_bounds__(GS_THREADS) k_cg_pre(const double2* __restrict__ zu, double2* __restrict__ W,
-                                                       CGState* __restrict__ st, int ib, int iter, int nkl, int NB,
-                                                       int NL, double Hxyz) {
-  __shared__ double sh[64];
-  __shared__ double part[8];
-  Grp g = grp_make(NL, part);
-  const int k = g.k;
-  const CGState st0 = st[k];
-  if (st0.done) return;  // uniform over the cluster, before any cluster-wide sum
-  const double2* base = zu + (size_t)k * NB * NL;
-  double2 *xk = wv(W, nkl, k, CG_XK, NL), *hxk = wv(W, nkl, k, CG_HXK, NL), *gk = wv(W, nkl, k, CG_GK, NL);
-  double2 *pk = wv(W, nkl, k, CG_PK, NL), *pko = wv(W, nkl, k, CG_PKO, NL);
-  const double xkHxk = st0.xkHxk;
-  GRP_FOR(i) gk[i] = make_double2(hxk[i].x - xkHxk * xk[i].x, hxk[i].y - xkHxk * xk[i].y);
-  for (int ibt = 0; ibt < ib; ++ibt) {
-    const double2* ut = base + (size_t)ibt * NL;
-    const double2 d = grp_zdot(g, ut, gk, sh);
-    const double2 zs = make_double2(d.x * Hxyz, d.y * Hxyz);
-    GRP_FOR(i) gk[i] = csub(gk[i], cmul(ut[i], zs));
+// x <- x - sum_j c_j u_j at one point
+__device__ __forceinline__ double2 cg_subtract(double2 x, const double2* __restrict__ u, int NL, int n,
+                                               const double2* c) {
+  int j = 0;
+  for (; j + 8 <= n; j += 8) {
+    double2 v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = u[(size_t)(j + q) * NL];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) x = csub(x, cmul(c[j + q], v[q]));
   }
-  const double s = grp_nrm2(g, gk, sh) * Hxyz;
-  if (iter == 1) {
-    GRP_FOR(i) pk[i] = gk[i];
-  } else {
-    const double uk = s / st0.gkgk;
-    GRP_FOR(i) pk[i] = make_double2(gk[i].x + uk * pk[i].x, gk[i].y + uk * pk[i].y);
+  for (; j < n; ++j) x = csub(x, cmul(c[j], u[(size_t)j * NL]));
+  return x;
+}
+
+// Hxyz <u_j|x> for n bands u_j into s.d, over the cluster (ends with a CTA barrier)
+__device__ __forceinline__ void grp_dots(Grp& g, const double2* __restrict__ u, int NL, int n, const double2* x,
+                                         double Hxyz) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  double2* loc = g.s->dots[g.dparity];
+  __syncthreads();  // x is written by other threads of the CTA
+  for (int j = warp; j < n; j += nw) {
+    const double2* uj = u + (size_t)j * NL;
+    double re = 0.0, im = 0.0;
+#pragma unroll 4
+    for (int i = g.lo + lane; i < g.hi; i += 32) zdot_add(re, im, uj[i], x[i]);
+    re = warp_sum_gs(re);
+    im = warp_sum_gs(im);
+    if (lane == 0) loc[j] = make_double2(re * Hxyz, im * Hxyz);
   }
-  const double2 d = grp_zdot(g, xk, pk, sh);
-  if (g.rank == 0 && threadIdx.x == 0) st[k].gkgk = s;
-  const double2 zs = make_double2(d.x * Hxyz, d.y * Hxyz);
-  GRP_FOR(i) pko[i] = csub(pk[i], cmul(xk[i], zs));
-  const double inv = 1.0 / sqrt(grp_nrm2(g, pko, sh) * Hxyz);
+  if (g.C > 1) cgx::this_cluster().sync(); else __syncthreads();
+  for (int j = threadIdx.x; j < n; j += blockDim.x) {
+    double2 t = make_double2(0.0, 0.0);
+    if (g.C > 1) {
+      cgx::cluster_group cl = cgx::this_cluster();
+      for (int r = 0; r < g.C; ++r) t = cadd(t, cl.map_shared_rank(loc, r)[j]);
+    } else {
+      t = loc[j];
+    }
+    g.s->d[j] = t;
+  }
+  __syncthreads();
+  g.dparity ^= 1;
+}
+
+// x <- x minus its projections on the ib lower bands, taken one by one
+template <bool REAL>
+__device__ __forceinline__ void grp_project(Grp& g, const CGArgs& a, int ib, double2* x) {
+  const double2* base = a.zu + (size_t)g.k * a.NB * a.NL;
+  for (int b0 = 0; b0 < ib; b0 += CGB) {
+    const int n = min(CGB, ib - b0);
+    const double2* u = base + (size_t)b0 * a.NL;
+    const size_t row = ((size_t)g.k * a.NB + b0) * CGB;
+    grp_dots(g, u, a.NL, n, x, a.Hxyz);
+    cg_solve<REAL>(a.M + row, a.MR + row, n, g.s->d, g.s->c);
+    __syncthreads();
+    GRP_FOR(i) x[i] = cg_subtract(x[i], u + i, a.NL, n, g.s->c);
+  }
+}
+
+// Row ib of (I + L)^-1 from the overlaps d_i = <u_i|u_ib> of the block's lower bands:
+// m = -l (I + L)^-1 with l_i = <u_ib|u_i> = conj(d_i), and 1 on the diagonal.  n = ib's
+// index in its block.
+__device__ __forceinline__ void cg_new_row(double2* __restrict__ M, double* __restrict__ MR, int n, const double2* d) {
+  for (int i = threadIdx.x; i <= n; i += blockDim.x) {
+    double2 m = make_double2(i == n ? 1.0 : 0.0, 0.0);
+    double mr = m.x;
+#pragma unroll 8
+    for (int l = i; l < n; ++l) {
+      m = csub(m, cmul(make_double2(d[l].x, -d[l].y), M[(size_t)l * CGB + i]));
+      mr = fma(-d[l].x, MR[(size_t)l * CGB + i], mr);
+    }
+    M[(size_t)n * CGB + i] = m;
+    MR[(size_t)n * CGB + i] = mr;
+  }
+}
+
+// gk = hxk - xkHxk xk (xkHxk = the new Rayleigh quotient); with pre: hk's start and T_band
+// are left to cg_after_gradient, once gk is orthogonal to the lower bands
+__device__ __forceinline__ void cg_gradient(Grp& g, const CGArgs& a, double e) {
+  const double2 *xk = wv(a.W, a.nkl, g.k, CG_XK, a.NL), *hxk = wv(a.W, a.nkl, g.k, CG_HXK, a.NL);
+  double2* gk = wv(a.W, a.nkl, g.k, CG_GK, a.NL);
+  GRP_FOR(i) gk[i] = make_double2(hxk[i].x - e * xk[i].x, hxk[i].y - e * xk[i].y);
+}
+
+// Conjugate direction from hk (the gradient gk itself without a preconditioner, else
+// K gk after its projections on the lower bands), pko = its normalised component
+// orthogonal to xk (CG.f90:92-106; with a preconditioner Payne et al., Rev. Mod. Phys.
+// 64, 1045 (1992), section V.B: hk orthogonal to xk too, beta = <gk|hk> / previous).
+// One exchange for every inner product (linear in the old direction), one for the norm.
+__device__ __forceinline__ void cg_direction(Grp& g, const CGArgs& a, bool pre, int iter, double gkgk_old) {
+  double2 *xk = wv(a.W, a.nkl, g.k, CG_XK, a.NL), *gk = wv(a.W, a.nkl, g.k, CG_GK, a.NL);
+  double2 *hk = pre ? wv(a.W, a.nkl, g.k, CG_HK, a.NL) : gk;
+  double2 *pk = wv(a.W, a.nkl, g.k, CG_PK, a.NL), *pko = wv(a.W, a.nkl, g.k, CG_PKO, a.NL);
+  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // <x|h>, Re <g|h>, <g|x>, <x|p_old>, <x|x>
+  GRP_FOR(i) {
+    const double2 x = xk[i], h = hk[i];
+    zdot_add(v[0], v[1], x, h);
+    if (pre) {
+      const double2 gg = gk[i];
+      v[2] = rdot(gg, h, v[2]);
+      zdot_add(v[3], v[4], gg, x);
+      v[7] = rdot(x, x, v[7]);
+    } else {
+      v[2] = rdot(h, h, v[2]);
+    }
+    if (iter > 1) zdot_add(v[5], v[6], x, pk[i]);
+  }
+  grp_allsum<8>(g, v);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] *= a.Hxyz;
+  double2 zs = make_double2(v[0], v[1]);     // <x|h>
+  double2 zh = make_double2(0.0, 0.0);       // the part of x taken out of h
+  double s = v[2];
+  if (pre) {  // h <- h - x <x|h>, s = Re <g|h>
+    zh = zs;
+    s -= v[3] * zh.x - v[4] * zh.y;
+    zs = make_double2(zs.x * (1.0 - v[7]), zs.y * (1.0 - v[7]));
+  }
+  const double uk = iter > 1 ? s / gkgk_old : 0.0;
+  if (iter > 1) zs = make_double2(fma(uk, v[5], zs.x), fma(uk, v[6], zs.y));
+  if (g.rank == 0 && threadIdx.x == 0) a.st[g.k].gkgk = s;
+  double n2[1] = {0.0};
+  GRP_FOR(i) {
+    const double2 x = xk[i];
+    double2 p = hk[i];
+    if (pre) p = csub(p, cmul(x, zh));
+    if (iter > 1) {
+      const double2 o = pk[i];
+      p = make_double2(fma(uk, o.x, p.x), fma(uk, o.y, p.y));
+    }
+    pk[i] = p;
+    p = csub(p, cmul(x, zs));
+    pko[i] = p;
+    n2[0] = rdot(p, p, n2[0]);
+  }
+  grp_allsum<1>(g, n2);
+  const double inv = 1.0 / sqrt(n2[0] * a.Hxyz);
   GRP_FOR(i) pko[i] = make_double2(pko[i].x * inv, pko[i].y * inv);
+}
+
+// hk starts as gk (the preconditioner works in place on it)
+__device__ __forceinline__ void cg_copy_gradient(Grp& g, const CGArgs& a) {
+  const double2* gk = wv(a.W, a.nkl, g.k, CG_GK, a.NL);
+  double2* hk = wv(a.W, a.nkl, g.k, CG_HK, a.NL);
+  GRP_FOR(i) hk[i] = gk[i];
+}
+
+// In the kernels below, proj: the projections on the lower bands run inside the
+// cluster; otherwise they are the separate kernels of launch_cg_project (few
+// k-points: the clusters alone would leave most SMs idle), and the kernel stops, or
+// starts, where they come.
+
+// The residual of the finished band ib-1, esp_var = sqrt(||H u - <u|H u> u||^2 Hxyz) occ
+// (CG.f90:124-126), then band ib orthogonalised against the lower bands with REAL
+// coefficients (s is real(8) in the reference, CG.f90:45,70) and normalised into xk.
+__global__ void __launch_bounds__(GS_THREADS) k_cg_open(const CGArgs a, int ib, int proj,
+                                                        const double* __restrict__ occ_gs,
+                                                        double* __restrict__ esp_var, double* __restrict__ res,
+                                                        int* __restrict__ iters) {
+  __shared__ GrpShared sm;
+  Grp g = grp_make(a.NL, &sm);
+  double2* xk = wv(a.W, a.nkl, g.k, CG_XK, a.NL);
+  if (ib > 0) {
+    const double2 *u = xk, *ht = wv(a.W, a.nkl, g.k, CG_HT, a.NL);
+    double e[1] = {0.0}, v[1] = {0.0};
+    GRP_FOR(i) e[0] = rdot(u[i], ht[i], e[0]);
+    grp_allsum<1>(g, e);
+    e[0] *= a.Hxyz;
+    GRP_FOR(i) {
+      const double2 r = make_double2(ht[i].x - e[0] * u[i].x, ht[i].y - e[0] * u[i].y);
+      v[0] = rdot(r, r, v[0]);
+    }
+    grp_allsum<1>(g, v);
+    if (g.rank == 0 && threadIdx.x == 0) {
+      const size_t o = (size_t)g.k * a.NB + ib - 1;
+      esp_var[o] = sqrt(v[0] * a.Hxyz) * occ_gs[o];
+      res[o] = sqrt(v[0] * a.Hxyz);  // the residual norm itself, for convergence tests
+      iters[o] = a.st[g.k].iters;
+    }
+  }
+  if (ib < a.NB) {
+    double2* u = a.zu + ((size_t)g.k * a.NB + ib) * a.NL;
+    if (proj) grp_project<true>(g, a, ib, u);
+    const double inv = 1.0 / sqrt(grp_nrm2(g, u) * a.Hxyz);
+    GRP_FOR(i) xk[i] = make_double2(u[i].x * inv, u[i].y * inv);
+    if (g.rank == 0 && threadIdx.x == 0) { a.st[g.k].done = 0; a.st[g.k].iters = 0; }
+  }
   grp_exit(g);
 }
 
-// Preconditioned variant (no reference counterpart; Payne et al., Rev. Mod.
-// Phys. 64, 1045 (1992), section V.B): the gradient gk (as above, orthogonal
-// to the lower bands) is preconditioned into hk = K gk by a separate kernel
-// chain; k_cg_dir orthogonalises hk against the lower bands and xk, and builds
-// the conjugate direction with beta = <gk|hk> / <gk|hk>_previous.
-// k_cg_grad also records the kinetic energy of xk (T_band, for the TPA form).
-__global__ void __launch_bounds__(GS_THREADS) k_cg_grad(const double2* __restrict__ zu, double2* __restrict__ W,
-                                                        CGState* __restrict__ st, double* __restrict__ tband, int ib,
-                                                        int nkl, int NB, int NL, double Hxyz) {
-  __shared__ double sh[64];
-  __shared__ double part[8];
-  Grp g = grp_make(NL, part);
-  const int k = g.k;
-  const CGState st0 = st[k];
-  if (st0.done) return;
-  const double2* base = zu + (size_t)k * NB * NL;
-  double2 *xk = wv(W, nkl, k, CG_XK, NL), *hxk = wv(W, nkl, k, CG_HXK, NL), *gk = wv(W, nkl, k, CG_GK, NL);
-  double2* hk = wv(W, nkl, k, CG_HK, NL);
-  const double xkHxk = st0.xkHxk;
-  GRP_FOR(i) gk[i] = make_double2(hxk[i].x - xkHxk * xk[i].x, hxk[i].y - xkHxk * xk[i].y);
-  for (int ibt = 0; ibt < ib; ++ibt) {
-    const double2* ut = base + (size_t)ibt * NL;
-    const double2 d = grp_zdot(g, ut, gk, sh);
-    const double2 zs = make_double2(d.x * Hxyz, d.y * Hxyz);
-    GRP_FOR(i) gk[i] = csub(gk[i], cmul(ut[i], zs));
-  }
-  GRP_FOR(i) hk[i] = gk[i];  // the preconditioner works in place on hk
-  const double t = grp_zdot(g, xk, wv(W, nkl, k, CG_TXK, NL), sh).x * Hxyz;
-  if (g.rank == 0 && threadIdx.x == 0) tband[k] = t;
-  grp_exit(g);
-}
-
-__global__ void __launch_bounds__(GS_THREADS) k_cg_dir(const double2* __restrict__ zu, double2* __restrict__ W,
-                                                       CGState* __restrict__ st, int ib, int iter, int nkl, int NB,
-                                                       int NL, double Hxyz) {
-  __shared__ double sh[64];
-  __shared__ double part[8];
-  Grp g = grp_make(NL, part);
-  const int k = g.k;
-  const CGState st0 = st[k];
-  if (st0.done) return;
-  const double2* base = zu + (size_t)k * NB * NL;
-  double2 *xk = wv(W, nkl, k, CG_XK, NL), *gk = wv(W, nkl, k, CG_GK, NL), *hk = wv(W, nkl, k, CG_HK, NL);
-  double2 *pk = wv(W, nkl, k, CG_PK, NL), *pko = wv(W, nkl, k, CG_PKO, NL);
-  for (int ibt = 0; ibt < ib; ++ibt) {
-    const double2* ut = base + (size_t)ibt * NL;
-    const double2 d = grp_zdot(g, ut, hk, sh);
-    const double2 zs = make_double2(d.x * Hxyz, d.y * Hxyz);
-    GRP_FOR(i) hk[i] = csub(hk[i], cmul(ut[i], zs));
-  }
-  {
-    const double2 d = grp_zdot(g, xk, hk, sh);
-    const double2 zs = make_double2(d.x * Hxyz, d.y * Hxyz);
-    GRP_FOR(i) hk[i] = csub(hk[i], cmul(xk[i], zs));
-  }
-  const double s = grp_zdot(g, gk, hk, sh).x * Hxyz;
-  if (iter == 1) {
-    GRP_FOR(i) pk[i] = hk[i];
-  } else {
-    const double uk = s / st0.gkgk;
-    GRP_FOR(i) pk[i] = make_double2(hk[i].x + uk * pk[i].x, hk[i].y + uk * pk[i].y);
-  }
-  const double2 d = grp_zdot(g, xk, pk, sh);
-  if (g.rank == 0 && threadIdx.x == 0) st[k].gkgk = s;
-  const double2 zs = make_double2(d.x * Hxyz, d.y * Hxyz);
-  GRP_FOR(i) pko[i] = csub(pk[i], cmul(xk[i], zs));
-  const double inv = 1.0 / sqrt(grp_nrm2(g, pko, sh) * Hxyz);
-  GRP_FOR(i) pko[i] = make_double2(pko[i].x * inv, pko[i].y * inv);
-  grp_exit(g);
-}
-
-// 2x2 Rayleigh-Ritz in span{xk, pko} and the update (CG.f90:108-119)
-__global__ void __launch_bounds__(GS_THREADS) k_cg_post(double2* __restrict__ W, CGState* __restrict__ st, int iter,
-                                                        int nkl, int NL, double Hxyz, double delta_cg) {
-  __shared__ double sh[64];
-  __shared__ double part[8];
-  Grp g = grp_make(NL, part);
-  const int k = g.k;
-  const CGState st0 = st[k];
-  if (st0.done) return;
-  double2 *xk = wv(W, nkl, k, CG_XK, NL), *hxk = wv(W, nkl, k, CG_HXK, NL), *txk = wv(W, nkl, k, CG_TXK, NL);
-  const double2 *pko = wv(W, nkl, k, CG_PKO, NL), *ht = wv(W, nkl, k, CG_HT, NL), *tt = wv(W, nkl, k, CG_TT, NL);
-  const double xkHxk = st0.xkHxk;
-  const double2 d1 = grp_zdot(g, xk, ht, sh);
-  const double2 xkHpk = make_double2(d1.x * Hxyz, d1.y * Hxyz);
-  const double pkHpk = grp_zdot(g, pko, ht, sh).x * Hxyz;
-  const double ev = 0.5 * ((xkHxk + pkHpk) - sqrt((xkHxk - pkHpk) * (xkHxk - pkHpk) +
-                                                 4 * (xkHpk.x * xkHpk.x + xkHpk.y * xkHpk.y)));
-  double2 cx = make_double2(xkHpk.x / (ev - xkHxk), xkHpk.y / (ev - xkHxk));
-  const double cp = 1.0 / sqrt(1.0 + (cx.x * cx.x + cx.y * cx.y));
-  cx = make_double2(cx.x * cp, cx.y * cp);
-  if (g.rank == 0 && threadIdx.x == 0) st[k].iters = iter;
-  if (fabs(ev - xkHxk) < delta_cg) {  // delta_cg = 1e-15 in the reference (CG.f90:42,114)
-    if (g.rank == 0 && threadIdx.x == 0) st[k].done = 1;
-    grp_exit(g);
-    return;
-  }
+// After H xk: the Rayleigh quotient, the gradient and (without a preconditioner) the
+// first direction (CG.f90:80-106).
+__global__ void __launch_bounds__(GS_THREADS) k_cg_first(const CGArgs a, int ib, int proj, int pre) {
+  __shared__ GrpShared sm;
+  Grp g = grp_make(a.NL, &sm);
+  const double2 *xk = wv(a.W, a.nkl, g.k, CG_XK, a.NL), *hxk = wv(a.W, a.nkl, g.k, CG_HXK, a.NL);
+  const double2* txk = wv(a.W, a.nkl, g.k, CG_TXK, a.NL);
+  double v[2] = {0.0, 0.0};
   GRP_FOR(i) {
-    xk[i] = cfma(cx, xk[i], make_double2(cp * pko[i].x, cp * pko[i].y));
-    hxk[i] = cfma(cx, hxk[i], make_double2(cp * ht[i].x, cp * ht[i].y));
-    txk[i] = cfma(cx, txk[i], make_double2(cp * tt[i].x, cp * tt[i].y));
+    v[0] = rdot(xk[i], hxk[i], v[0]);
+    if (pre) v[1] = rdot(xk[i], txk[i], v[1]);
   }
-  const double x2 = grp_zdot(g, xk, hxk, sh).x * Hxyz;
-  if (g.rank == 0 && threadIdx.x == 0) st[k].xkHxk = x2;
-  grp_exit(g);
-}
-
-// zu(:,ib) = xk / |xk|; the normalised band is also left in xk for the residual
-__global__ void __launch_bounds__(GS_THREADS) k_cg_end(double2* __restrict__ zu, double2* __restrict__ W, int ib,
-                                                       int nkl, int NB, int NL, double Hxyz) {
-  __shared__ double sh[64];
-  __shared__ double part[8];
-  Grp g = grp_make(NL, part);
-  const int k = g.k;
-  double2* xk = wv(W, nkl, k, CG_XK, NL);
-  double2* u = zu + ((size_t)k * NB + ib) * NL;
-  const double inv = 1.0 / sqrt(grp_nrm2(g, xk, sh) * Hxyz);
-  GRP_FOR(i) {
-    const double2 v = make_double2(xk[i].x * inv, xk[i].y * inv);
-    u[i] = v;
-    xk[i] = v;
-  }
-  grp_exit(g);
-}
-
-// esp_var(ib,k) = sqrt(||H u - <u|H u> u||^2 Hxyz) occ(ib,k)  (CG.f90:124-126)
-__global__ void __launch_bounds__(GS_THREADS) k_cg_resid(double2* __restrict__ W, const double* __restrict__ occ_gs,
-                                                         double* __restrict__ esp_var, double* __restrict__ res,
-                                                         int ib, int nkl, int NB, int NL, double Hxyz) {
-  __shared__ double sh[64];
-  __shared__ double part[8];
-  Grp g = grp_make(NL, part);
-  const int k = g.k;
-  const double2 *u = wv(W, nkl, k, CG_XK, NL), *ht = wv(W, nkl, k, CG_HT, NL);
-  const double e = grp_zdot(g, u, ht, sh).x * Hxyz;
-  double v[1] = {0.0};
-  GRP_FOR(i) {
-    const double2 r = make_double2(ht[i].x - e * u[i].x, ht[i].y - e * u[i].y);
-    v[0] = fma(r.x, r.x, fma(r.y, r.y, v[0]));
-  }
-  grp_allsum<1>(g, v, sh);
+  grp_allsum<2>(g, v);
+  const double e = v[0] * a.Hxyz;
   if (g.rank == 0 && threadIdx.x == 0) {
-    esp_var[(size_t)k * NB + ib] = sqrt(v[0] * Hxyz) * occ_gs[(size_t)k * NB + ib];
-    res[(size_t)k * NB + ib] = sqrt(v[0] * Hxyz);  // the residual norm itself, for convergence tests
+    a.st[g.k].xkHxk = e;
+    if (pre) a.tband[g.k] = v[1] * a.Hxyz;
+  }
+  cg_gradient(g, a, e);
+  if (proj) {
+    grp_project<false>(g, a, ib, wv(a.W, a.nkl, g.k, CG_GK, a.NL));
+    if (pre) cg_copy_gradient(g, a);
+    else cg_direction(g, a, false, 1, 0.0);
   }
   grp_exit(g);
+}
+
+// The direction of iteration iter from the projected gradient (or, with a
+// preconditioner, from hk).
+__global__ void __launch_bounds__(GS_THREADS) k_cg_dir(const CGArgs a, int ib, int iter, int proj, int pre) {
+  __shared__ GrpShared sm;
+  Grp g = grp_make(a.NL, &sm);
+  const CGState st0 = a.st[g.k];
+  if (st0.done) return;  // uniform over the cluster, before any cluster-wide sum
+  if (pre && proj) grp_project<false>(g, a, ib, wv(a.W, a.nkl, g.k, CG_HK, a.NL));
+  cg_direction(g, a, pre, iter, st0.gkgk);
+  grp_exit(g);
+}
+
+// 2x2 Rayleigh-Ritz in span{xk, pko} and the update (CG.f90:108-119); then, as long as
+// iterations are left, the next gradient (and direction), else the finished band:
+// zu(:,ib) = xk / |xk|, also left in xk for the residual, and its row of (I + L)^-1.
+__global__ void __launch_bounds__(GS_THREADS) k_cg_step(const CGArgs a, int ib, int iter, int last, int proj, int pre,
+                                                        double delta_cg) {
+  __shared__ GrpShared sm;
+  Grp g = grp_make(a.NL, &sm);
+  const int k = g.k;
+  const CGState st0 = a.st[k];
+  double2 *xk = wv(a.W, a.nkl, k, CG_XK, a.NL), *hxk = wv(a.W, a.nkl, k, CG_HXK, a.NL);
+  double2* txk = wv(a.W, a.nkl, k, CG_TXK, a.NL);
+  bool done = st0.done != 0;
+  if (!done) {
+    const double2 *pko = wv(a.W, a.nkl, k, CG_PKO, a.NL), *ht = wv(a.W, a.nkl, k, CG_HT, a.NL);
+    const double2* tt = wv(a.W, a.nkl, k, CG_TT, a.NL);
+    const double xkHxk = st0.xkHxk;
+    double v[3] = {0.0, 0.0, 0.0};
+    GRP_FOR(i) {
+      const double2 h = ht[i];
+      zdot_add(v[0], v[1], xk[i], h);
+      v[2] = rdot(pko[i], h, v[2]);
+    }
+    grp_allsum<3>(g, v);
+    const double2 xkHpk = make_double2(v[0] * a.Hxyz, v[1] * a.Hxyz);
+    const double pkHpk = v[2] * a.Hxyz;
+    const double ev = 0.5 * ((xkHxk + pkHpk) - sqrt((xkHxk - pkHpk) * (xkHxk - pkHpk) +
+                                                   4 * (xkHpk.x * xkHpk.x + xkHpk.y * xkHpk.y)));
+    double2 cx = make_double2(xkHpk.x / (ev - xkHxk), xkHpk.y / (ev - xkHxk));
+    const double cp = 1.0 / sqrt(1.0 + (cx.x * cx.x + cx.y * cx.y));
+    cx = make_double2(cx.x * cp, cx.y * cp);
+    if (g.rank == 0 && threadIdx.x == 0) a.st[k].iters = iter;
+    if (fabs(ev - xkHxk) < delta_cg) {  // delta_cg = 1e-15 in the reference (CG.f90:42,114)
+      done = true;
+      if (g.rank == 0 && threadIdx.x == 0) a.st[k].done = 1;
+    } else {
+      double w[2] = {0.0, 0.0};
+      GRP_FOR(i) {
+        const double2 p = pko[i], h = ht[i], t = tt[i];
+        const double2 x = cfma(cx, xk[i], make_double2(cp * p.x, cp * p.y));
+        const double2 hx = cfma(cx, hxk[i], make_double2(cp * h.x, cp * h.y));
+        const double2 tx = cfma(cx, txk[i], make_double2(cp * t.x, cp * t.y));
+        xk[i] = x;
+        hxk[i] = hx;
+        txk[i] = tx;
+        w[0] = rdot(x, hx, w[0]);
+        w[1] = rdot(x, tx, w[1]);
+      }
+      if (!last) {
+        grp_allsum<2>(g, w);
+        const double e = w[0] * a.Hxyz;
+        if (g.rank == 0 && threadIdx.x == 0) {
+          a.st[k].xkHxk = e;
+          if (pre) a.tband[k] = w[1] * a.Hxyz;
+        }
+        cg_gradient(g, a, e);
+        if (proj) {
+          grp_project<false>(g, a, ib, wv(a.W, a.nkl, k, CG_GK, a.NL));
+          if (pre) cg_copy_gradient(g, a);
+          else cg_direction(g, a, false, iter + 1, st0.gkgk);
+        }
+      }
+    }
+  }
+  if (last) {
+    double2* u = a.zu + ((size_t)k * a.NB + ib) * a.NL;
+    const double inv = 1.0 / sqrt(grp_nrm2(g, xk) * a.Hxyz);
+    GRP_FOR(i) {
+      const double2 x = make_double2(xk[i].x * inv, xk[i].y * inv);
+      u[i] = x;
+      xk[i] = x;
+    }
+    if (proj) {
+      const int b0 = ib / CGB * CGB;
+      grp_dots(g, a.zu + ((size_t)k * a.NB + b0) * a.NL, a.NL, ib - b0, u, a.Hxyz);
+      const size_t row = ((size_t)k * a.NB + b0) * CGB;
+      if (g.rank == 0) cg_new_row(a.M + row, a.MR + row, ib - b0, g.s->d);
+    }
+  }
+  grp_exit(g);
+}
+
+// ------------------------------------------- projections over the whole GPU --
+// Few k-points: nkl clusters of at most 16 CTAs leave most SMs idle while they read
+// the lower bands twice per projection.  Here the inner products run over (k-point,
+// CG_DB bands, range of points) and the subtraction over (k-point, 256 points).
+constexpr int CG_DB = 4;  // bands of a CTA, sharing the loads of x
+
+__global__ void __launch_bounds__(256) k_cg_dots(const double2* __restrict__ zu, const double2* __restrict__ x,
+                                                 size_t xstride, int b0, int n, int NB, int NL, int chunk,
+                                                 const CGState* __restrict__ st, double2* __restrict__ part) {
+  __shared__ double sh[32 * 2 * CG_DB];
+  const int k = blockIdx.z, j0 = blockIdx.x * CG_DB, sp = blockIdx.y;
+  if (st && st[k].done) return;
+  const double2* u = zu + ((size_t)k * NB + b0 + j0) * NL;
+  const double2* xk = x + k * xstride;
+  const int nj = min(CG_DB, n - j0), i1 = min(NL, (sp + 1) * chunk);
+  double v[2 * CG_DB];
+#pragma unroll
+  for (int j = 0; j < 2 * CG_DB; ++j) v[j] = 0.0;
+#pragma unroll 2
+  for (int i = sp * chunk + threadIdx.x; i < i1; i += 256) {
+    const double2 xi = xk[i];
+#pragma unroll
+    for (int j = 0; j < CG_DB; ++j)
+      if (j < nj) zdot_add(v[2 * j], v[2 * j + 1], u[(size_t)j * NL + i], xi);
+  }
+  block_allsum<2 * CG_DB>(v, sh);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int j = 0; j < CG_DB; ++j)
+      if (j < nj) part[((size_t)k * gridDim.y + sp) * CGB + j0 + j] = make_double2(v[2 * j], v[2 * j + 1]);
+}
+
+// d_j = Hxyz sum over the ranges, in order
+__device__ __forceinline__ void cg_sum_dots(const double2* __restrict__ part, int k, int nsplit, int n, double Hxyz,
+                                            double2* d) {
+  for (int j = threadIdx.x; j < n; j += blockDim.x) {
+    double2 t = make_double2(0.0, 0.0);
+    for (int sp = 0; sp < nsplit; ++sp) t = cadd(t, part[((size_t)k * nsplit + sp) * CGB + j]);
+    d[j] = make_double2(t.x * Hxyz, t.y * Hxyz);
+  }
+}
+
+template <bool REAL>
+__global__ void __launch_bounds__(256) k_cg_subtract(const double2* __restrict__ zu, double2* __restrict__ x,
+                                                     size_t xstride, double2* __restrict__ copy, int b0, int n, int NB,
+                                                     int NL, double Hxyz, const double2* __restrict__ M,
+                                                     const double* __restrict__ MR, const CGState* __restrict__ st,
+                                                     const double2* __restrict__ part, int nsplit) {
+  __shared__ double2 d[CGB], c[CGB];
+  const int k = blockIdx.y;
+  if (st && st[k].done) return;
+  cg_sum_dots(part, k, nsplit, n, Hxyz, d);
+  __syncthreads();
+  const size_t row = ((size_t)k * NB + b0) * CGB;
+  cg_solve<REAL>(M + row, MR + row, n, d, c);
+  __syncthreads();
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= NL) return;
+  const double2 v = cg_subtract(x[k * xstride + i], zu + ((size_t)k * NB + b0) * NL + i, NL, n, c);
+  x[k * xstride + i] = v;
+  if (copy) copy[(size_t)k * NL + i] = v;
+}
+
+__global__ void __launch_bounds__(256) k_cg_row(double2* __restrict__ M, double* __restrict__ MR, int b0, int n, int NB,
+                                                double Hxyz, const double2* __restrict__ part, int nsplit) {
+  __shared__ double2 d[CGB];
+  const int k = blockIdx.x;
+  cg_sum_dots(part, k, nsplit, n, Hxyz, d);
+  __syncthreads();
+  const size_t row = ((size_t)k * NB + b0) * CGB;
+  cg_new_row(M + row, MR + row, n, d);
 }
 
 // ------------------------------------------------------------------ launch --
@@ -397,116 +624,123 @@ static cudaError_t launch_gs(const System& s, Kern kern, Args... args) {
   }
 }
 
-cudaError_t launch_gram_schmidt(const System& s, double2* zu) {
-  return launch_gs(s, k_gram_schmidt, zu, s.NB, s.NL, s.Hxyz);
+cudaError_t launch_gram_schmidt_panel(const System& s, double2* zu, int p0, int pb, const int* bad) {
+  return launch_gs(s, k_gram_schmidt, zu, s.NB, s.NL, s.Hxyz, p0, pb, bad);
 }
-cudaError_t launch_cg_begin(const System& s, double2* zu, double2* W, void* st, int ib) {
-  return launch_gs(s, k_cg_begin, zu, W, (CGState*)st, ib, s.nkl, s.NB, s.NL, s.Hxyz);
+
+static CGArgs cg_args(const System& s, double2* zu) {
+  CGArgs a;
+  a.zu = zu;
+  a.W = s.gs_W;
+  a.st = (CGState*)s.gs_st;
+  a.M = s.gs_M;
+  a.MR = s.gs_MR;
+  a.tband = s.gs_tb;
+  a.nkl = s.nkl;
+  a.NB = s.NB;
+  a.NL = s.NL;
+  a.Hxyz = s.Hxyz;
+  return a;
 }
-cudaError_t launch_cg_dot0(const System& s, double2* W, void* st) {
-  return launch_gs(s, k_cg_dot0, W, (CGState*)st, s.nkl, s.NL, s.Hxyz);
+
+// Where the lower bands are projected: inside the clusters, or, when these cover less
+// than half the SMs and a CTA's share of the lower bands takes longer to read than two
+// more launches, by the kernels over the whole GPU.
+bool cg_wide(const System& s) {
+  const int C = gs_cluster_size(s);
+  return 2 * s.nkl * C < s.nsm && (size_t)s.NL / C * s.NB >= 131072;
 }
-cudaError_t launch_cg_pre(const System& s, const double2* zu, double2* W, void* st, int ib, int iter) {
-  return launch_gs(s, k_cg_pre, zu, W, (CGState*)st, ib, iter, s.nkl, s.NB, s.NL, s.Hxyz);
+
+static int cg_splits(const System& s, int n) {
+  const int ctas = s.nkl * ((n + CG_DB - 1) / CG_DB);
+  return std::max(1, std::min({CG_DOT_SPLITS, (4 * s.nsm + ctas - 1) / ctas, (s.NL + 1023) / 1024}));
 }
-cudaError_t launch_cg_post(const System& s, double2* W, void* st, int iter) {
-  return launch_gs(s, k_cg_post, W, (CGState*)st, iter, s.nkl, s.NL, s.Hxyz, s.cg_delta);
+
+static cudaError_t launch_cg_dots(const System& s, const double2* zu, const double2* x, size_t xstride, int b0, int n,
+                                  const CGState* st, int& nsplit) {
+  nsplit = cg_splits(s, n);
+  const int chunk = (s.NL + nsplit - 1) / nsplit;
+  k_cg_dots<<<dim3((n + CG_DB - 1) / CG_DB, nsplit, s.nkl), 256, 0, s.launch_stream()>>>(zu, x, xstride, b0, n, s.NB,
+                                                                                        s.NL, chunk, st, s.gs_dots);
+  return cudaGetLastError();
 }
-cudaError_t launch_cg_end(const System& s, double2* zu, double2* W, int ib) {
-  return launch_gs(s, k_cg_end, zu, W, ib, s.nkl, s.NB, s.NL, s.Hxyz);
+
+// which: the work vector (CG_GK: also copied to hk if copy_hk), or -1 for band ib of zu
+// itself, with the real coefficients
+cudaError_t launch_cg_project(const System& s, double2* zu, int ib, int which, bool copy_hk) {
+  double2* x = which < 0 ? zu + (size_t)ib * s.NL : s.gs_W + (size_t)which * s.nkl * s.NL;
+  const size_t xs = which < 0 ? (size_t)s.NB * s.NL : (size_t)s.NL;
+  const CGState* st = which < 0 ? nullptr : (const CGState*)s.gs_st;
+  double2* copy = copy_hk ? s.gs_W + (size_t)CG_HK * s.nkl * s.NL : nullptr;
+  if (ib == 0 && copy)
+    return cudaMemcpyAsync(copy, x, (size_t)s.nkl * s.NL * sizeof(double2), cudaMemcpyDeviceToDevice, s.stream);
+  for (int b0 = 0; b0 < ib; b0 += CGB) {
+    const int n = std::min(CGB, ib - b0);
+    int ns = 1;
+    cudaError_t e = launch_cg_dots(s, zu, x, xs, b0, n, st, ns);
+    if (e != cudaSuccess) return e;
+    const dim3 grid((s.NL + 255) / 256, s.nkl);
+    double2* cp = b0 + n == ib ? copy : nullptr;
+    if (which < 0)
+      k_cg_subtract<true><<<grid, 256, 0, s.launch_stream()>>>(zu, x, xs, cp, b0, n, s.NB, s.NL, s.Hxyz, s.gs_M,
+                                                               s.gs_MR, st, s.gs_dots, ns);
+    else
+      k_cg_subtract<false><<<grid, 256, 0, s.launch_stream()>>>(zu, x, xs, cp, b0, n, s.NB, s.NL, s.Hxyz, s.gs_M,
+                                                                s.gs_MR, st, s.gs_dots, ns);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
-cudaError_t launch_cg_grad(const System& s, const double2* zu, double2* W, void* st, double* tband, int ib) {
-  return launch_gs(s, k_cg_grad, zu, W, (CGState*)st, tband, ib, s.nkl, s.NB, s.NL, s.Hxyz);
+
+// the finished band's row of (I + L)^-1 (wide form; the cluster form does it in k_cg_step)
+cudaError_t launch_cg_row(const System& s, double2* zu, int ib) {
+  const int b0 = ib / CGB * CGB, n = ib - b0;
+  int ns = 1;
+  if (n > 0) {
+    const cudaError_t e = launch_cg_dots(s, zu, zu + (size_t)ib * s.NL, (size_t)s.NB * s.NL, b0, n, nullptr, ns);
+    if (e != cudaSuccess) return e;
+  }
+  k_cg_row<<<s.nkl, 256, 0, s.launch_stream()>>>(s.gs_M, s.gs_MR, b0, n, s.NB, s.Hxyz, s.gs_dots, ns);
+  return cudaGetLastError();
 }
-cudaError_t launch_cg_dir(const System& s, const double2* zu, double2* W, void* st, int ib, int iter) {
-  return launch_gs(s, k_cg_dir, zu, W, (CGState*)st, ib, iter, s.nkl, s.NB, s.NL, s.Hxyz);
+
+cudaError_t launch_cg_open(const System& s, double2* zu, int ib, bool proj) {
+  return launch_gs(s, k_cg_open, cg_args(s, zu), ib, proj ? 1 : 0, (const double*)s.occ_gs, s.gs_out, s.gs_res,
+                   s.gs_iters);
 }
-cudaError_t launch_cg_resid(const System& s, double2* W, const double* occ_gs, double* esp_var, double* res, int ib) {
-  return launch_gs(s, k_cg_resid, W, occ_gs, esp_var, res, ib, s.nkl, s.NB, s.NL, s.Hxyz);
+cudaError_t launch_cg_first(const System& s, double2* zu, int ib, bool proj, bool pre) {
+  return launch_gs(s, k_cg_first, cg_args(s, zu), ib, proj ? 1 : 0, pre ? 1 : 0);
+}
+cudaError_t launch_cg_dir(const System& s, double2* zu, int ib, int iter, bool proj, bool pre) {
+  return launch_gs(s, k_cg_dir, cg_args(s, zu), ib, iter, proj ? 1 : 0, pre ? 1 : 0);
+}
+cudaError_t launch_cg_step(const System& s, double2* zu, int ib, int iter, bool last, bool proj, bool pre) {
+  return launch_gs(s, k_cg_step, cg_args(s, zu), ib, iter, last ? 1 : 0, proj ? 1 : 0, pre ? 1 : 0, s.cg_delta);
 }
 size_t cg_state_bytes() { return sizeof(CGState); }
 int cg_work_vectors() { return CG_NW; }
 
-// ------------------------------------------------------ subspace H (ZGEMM) --
-// part[sp][k][n][m] = sum_{i in split sp} conj(A[k][m][i]) B[k][n][i]
-// A, B: [k][NB][NL].  16x16 output tile per CTA, K split over blockIdx.z.
-constexpr int GT = 16, GK = 32;
-
-__global__ void __launch_bounds__(GT * GT) k_zgemm_hn(const double2* __restrict__ A, const double2* __restrict__ B,
-                                                     int NB, int NL, int kchunk, double2* __restrict__ part) {
-  __shared__ double2 sa[GT][GK + 1], sb[GT][GK + 1];
-  const int k = blockIdx.x / ((NB + GT - 1) / GT);
-  const int tm = blockIdx.x % ((NB + GT - 1) / GT), tn = blockIdx.y;
-  const int sp = blockIdx.z;
-  const int tx = threadIdx.x % GT, ty = threadIdx.x / GT;
-  const int m = tm * GT + tx, n = tn * GT + ty;
-  const int i0 = sp * kchunk, i1 = min(i0 + kchunk, NL);
-  const double2* Ak = A + (size_t)k * NB * NL;
-  const double2* Bk = B + (size_t)k * NB * NL;
-  double2 acc = make_double2(0, 0);
-  for (int ib = i0; ib < i1; ib += GK) {
-    for (int e = threadIdx.x; e < GT * GK; e += GT * GT) {
-      const int r = e / GK, c = e % GK, i = ib + c;
-      const int mr = tm * GT + r, nr = tn * GT + r;
-      sa[r][c] = (mr < NB && i < i1) ? Ak[(size_t)mr * NL + i] : make_double2(0, 0);
-      sb[r][c] = (nr < NB && i < i1) ? Bk[(size_t)nr * NL + i] : make_double2(0, 0);
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int c = 0; c < GK; ++c) acc = cfmaj(sa[tx][c], sb[ty][c], acc);
-    __syncthreads();
-  }
-  const int nkl = gridDim.x / ((NB + GT - 1) / GT);
-  if (m < NB && n < NB) part[(((size_t)sp * nkl + k) * NB + n) * NB + m] = acc;
-}
-
-// za[k][n][m] = Hxyz * sum_sp part[sp][k][n][m]  then made Hermitian like
-// diag_omp builds it (GS/diag.f90:112-116): the lower triangle (m > n) is
-// computed, the upper is its conjugate, the diagonal is real.
-__global__ void k_zgemm_reduce_herm(const double2* __restrict__ part, int nsplit, int nkl, int NB, double Hxyz,
-                                    double2* __restrict__ za) {
-  const size_t tot = (size_t)nkl * NB * NB;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < tot; e += (size_t)gridDim.x * blockDim.x) {
-    const int k = (int)(e / ((size_t)NB * NB));
-    const int n = (int)((e / NB) % NB), m = (int)(e % NB);
-    // element (row m, column n) of za(:,:) stored at za[k][n][m] (column-major)
-    const int lo_r = m > n ? m : n, lo_c = m > n ? n : m;  // lower-triangle source
-    double2 s = make_double2(0, 0);
-    for (int sp = 0; sp < nsplit; ++sp) {
-      const double2 p = part[(((size_t)sp * nkl + k) * NB + lo_c) * NB + lo_r];
-      s.x += p.x;
-      s.y += p.y;
-    }
-    s = make_double2(s.x * Hxyz, s.y * Hxyz);
-    if (m == n) s.y = 0.0;
-    else if (m < n) s.y = -s.y;
-    za[e] = s;
-  }
-}
-
-cudaError_t launch_subspace_h(const System& s, const double2* U, const double2* HU, double2* part, int nsplit,
-                              double2* za) {
-  const int nt = (s.NB + GT - 1) / GT;
-  const int kchunk = ((s.NL + nsplit - 1) / nsplit + GK - 1) / GK * GK;
-  dim3 grid(s.nkl * nt, nt, nsplit);
-  k_zgemm_hn<<<grid, GT * GT, 0, s.launch_stream()>>>(U, HU, s.NB, s.NL, kchunk, part);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  const size_t tot = (size_t)s.nkl * s.NB * s.NB;
-  k_zgemm_reduce_herm<<<(int)std::min<size_t>((tot + 255) / 256, 4096), 256, 0, s.launch_stream()>>>(part, nsplit, s.nkl, s.NB,
-                                                                                             s.Hxyz, za);
-  return cudaGetLastError();
-}
-
 // ------------------------------------------- Hermitian Jacobi eigensolver --
 // Cyclic two-sided Jacobi with the round-robin ordering: each step rotates
-// n/2 disjoint index pairs at once (rows, then columns, then the eigenvector
-// columns).  For a pair (p,q) with A_pq = |b| e^{i phi}, J = D R with
-// D = diag(1, e^{-i phi}) (makes the pair real) and the real Jacobi rotation
-// R = [[c, s], [-s, c]], t = sign(tau)/(|tau|+sqrt(1+tau^2)), tau = (a_qq-a_pp)/(2|b|).
-// One CTA per k-point; A and V (column-major, [k][col][row]) live in global memory.
-// Sweeps stop when the off-diagonal norm is below 1e-15 of the Frobenius norm,
-// or after max_sweeps (the count used is written to sweeps[k]).
+// n/2 disjoint index pairs at once.  For a pair (p,q) with A_pq = |b| e^{i phi},
+// J = D R with D = diag(1, e^{-i phi}) (makes the pair real) and the real Jacobi
+// rotation R = [[c, s], [-s, c]], t = sign(tau)/(|tau|+sqrt(1+tau^2)),
+// tau = (a_qq-a_pp)/(2|b|).
+//
+// One CTA per k-point.  The 2x2 blocks (pair, pair) of A <- J^H A J and the pairs of
+// columns of V <- V J are independent, so a step is one sweep over them between two
+// barriers; A and V live in shared memory as long as both fit (JAC_SMEM), else in
+// global memory.  Bound by the chain of FP64 square roots and divisions of the next
+// step's rotations and the two barriers.
+// At 32 k-points x 40 bands: 1.05 ms with rows and columns rotated one after the
+// other in global memory; the time now stands at launch_jacobi.
+//
+// Sweeps stop when the off-diagonal norm of the upper triangle, the one the rotations
+// are taken from, is below 1e-15 of the Frobenius norm, or after max_sweeps (the count
+// used is written to sweeps[k]).  (Rounding leaves the lower triangle a floor of its own
+// that the sweeps do not lower, at 128 bands above that threshold.)  Pairs below 1e-25 of
+// the norm are not rotated: in the square of a tiny A_pq an underflow would make e^{i phi}
+// a number of another modulus, and the rotation no rotation.
 __device__ __forceinline__ int rr_partner(int i, int step, int n) {
   // round-robin: position 0 fixed, others rotate; returns the partner of index i
   if (i == 0) return 1 + (step % (n - 1));
@@ -519,146 +753,149 @@ __device__ __forceinline__ int rr_partner(int i, int step, int n) {
   return idx + 1;
 }
 
+
+struct JacPair {
+  int p, q;            // q = -1: the odd index out
+  double c, s;
+  double2 eph;         // e^{i phi}
+};
+
+constexpr size_t JAC_SMEM = 220 * 1024;
+
+static size_t jac_pair_bytes(int NB) { return (size_t)((NB + 1) / 2) * sizeof(JacPair) + (size_t)NB * (sizeof(double) + sizeof(int)); }
+
 __global__ void __launch_bounds__(1024) k_jacobi_herm(double2* __restrict__ Aall, double2* __restrict__ Vall, int NB,
-                                                      int max_sweeps, double* __restrict__ w, int* __restrict__ sweeps) {
-  extern __shared__ double jsh[];
-  // rotation parameters per index (owner p < q): c, s, cos(phi), sin(phi), partner
-  double* cs = jsh;                      // [NB] c of the pair owned by p
-  double* sn = cs + NB;                  // [NB] s
-  double* ph_c = sn + NB;                // [NB] cos(phi)
-  double* ph_s = ph_c + NB;              // [NB] sin(phi)
-  int* partner = (int*)(ph_s + NB);      // [NB]
+                                                      int max_sweeps, int in_smem, double* __restrict__ w,
+                                                      int* __restrict__ sweeps) {
+  extern __shared__ __align__(16) unsigned char jraw[];
+  const int n = NB + (NB & 1), nh = n / 2;  // even count for the round-robin (index NB is a dummy)
+  JacPair* pr = reinterpret_cast<JacPair*>(jraw);           // [nh]
+  double* ev = reinterpret_cast<double*>(pr + nh);          // [NB] eigenvalues
+  int* rank = reinterpret_cast<int*>(ev + NB);              // [NB]
+  double2* mats = reinterpret_cast<double2*>(jraw + (((size_t)((unsigned char*)(rank + NB) - jraw) + 15) & ~(size_t)15));
   __shared__ double sh[64];
-  __shared__ int s_conv;
-  const int k = blockIdx.x;
-  double2* A = Aall + (size_t)k * NB * NB;
-  double2* V = Vall + (size_t)k * NB * NB;
+  const int k = blockIdx.x, t = threadIdx.x, nt = blockDim.x;
+  double2* Ag = Aall + (size_t)k * NB * NB;
+  double2* Vg = Vall + (size_t)k * NB * NB;
+  double2* A = in_smem ? mats : Ag;
+  double2* V = in_smem ? mats + (size_t)NB * NB : Vg;
 #define AE(r, c) A[(size_t)(c) * NB + (r)]
 #define VE(r, c) V[(size_t)(c) * NB + (r)]
-  for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) VE(e % NB, e / NB) = make_double2((e % NB) == (e / NB) ? 1.0 : 0.0, 0.0);
-  const int n = NB + (NB & 1);  // even count for the round-robin (index NB is a dummy)
+  for (int e = t; e < NB * NB; e += nt) {
+    if (in_smem) A[e] = Ag[e];
+    V[e] = make_double2((e % NB) == (e / NB) ? 1.0 : 0.0, 0.0);
+  }
+  __syncthreads();
   int sweep = 0;
   for (; sweep < max_sweeps; ++sweep) {
-    // convergence test
-    double v[2] = {0.0, 0.0};
-    for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
+    double v[2] = {0.0, 0.0};  // squared norms: the diagonal, the upper triangle
+    for (int e = t; e < NB * NB; e += nt) {
       const int r = e % NB, c = e / NB;
-      const double2 x = AE(r, c);
-      const double m2 = x.x * x.x + x.y * x.y;
-      v[0] += m2;
-      if (r != c) v[1] += m2;
+      const double2 x = A[e];
+      if (r <= c) v[r != c] += x.x * x.x + x.y * x.y;
     }
-    block_allsum<2>(v, sh);
-    if (threadIdx.x == 0) s_conv = (v[1] <= 1e-30 * v[0]) ? 1 : 0;
-    __syncthreads();
-    if (s_conv) break;
+    block_allsum<2>(v, sh);  // the same in every thread
+    const double fro2 = v[0] + 2.0 * v[1];
+    if (2.0 * v[1] <= 1e-30 * fro2) break;
+    const double tiny2 = 1e-50 * fro2;
     for (int step = 0; step < n - 1; ++step) {
-      for (int p = threadIdx.x; p < NB; p += blockDim.x) {
-        const int q = rr_partner(p, step, n);
-        partner[p] = q < NB ? q : -1;
-        cs[p] = 1.0; sn[p] = 0.0; ph_c[p] = 1.0; ph_s[p] = 0.0;
-        if (q < NB && p < q) {
-          const double app = AE(p, p).x, aqq = AE(q, q).x;
-          const double2 b = AE(p, q);
-          const double ab = sqrt(b.x * b.x + b.y * b.y);
-          if (ab > 0.0) {
+      for (int i = t; i < nh; i += nt) {
+        // ring position i pairs with n-1-i (i = 0: the fixed index)
+        const int q0 = i == 0 ? 0 : 1 + (i + step) % (n - 1), q1 = rr_partner(q0, step, n);
+        JacPair j;
+        j.p = min(q0, q1);
+        j.q = max(q0, q1) < NB ? max(q0, q1) : -1;
+        j.c = 1.0;
+        j.s = 0.0;
+        j.eph = make_double2(1.0, 0.0);
+        if (j.q >= 0) {
+          const double app = AE(j.p, j.p).x, aqq = AE(j.q, j.q).x;
+          const double2 b = AE(j.p, j.q);
+          const double m2 = b.x * b.x + b.y * b.y;
+          if (m2 > tiny2 && m2 > 1e-290) {
+            const double ab = sqrt(m2);
             const double tau = (aqq - app) / (2.0 * ab);
-            const double t = (tau >= 0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-            const double c = 1.0 / sqrt(1.0 + t * t);
-            cs[p] = c; sn[p] = t * c; ph_c[p] = b.x / ab; ph_s[p] = b.y / ab;
+            const double tt = (tau >= 0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
+            j.c = 1.0 / sqrt(1.0 + tt * tt);
+            j.s = tt * j.c;
+            j.eph = make_double2(b.x / ab, b.y / ab);
+          }
+        }
+        pr[i] = j;
+      }
+      __syncthreads();
+      // A <- J^H A J, block by block; V <- V J, row by row
+      for (int e = t; e < nh * nh + nh * NB; e += nt) {
+        if (e < nh * nh) {
+          const JacPair a = pr[e % nh], b = pr[e / nh];
+          const int rows[2] = {a.p, a.q}, cols[2] = {b.p, b.q};
+          double2 x[2][2];
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+              x[i][j] = rows[i] >= 0 && cols[j] >= 0 ? AE(rows[i], cols[j]) : make_double2(0.0, 0.0);
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {  // rows: new_p = c x_p - s e^{i phi} x_q, new_q = s x_p + c e^{i phi} x_q
+            const double2 ex = cmul(a.eph, x[1][j]), xp = x[0][j];
+            x[0][j] = make_double2(a.c * xp.x - a.s * ex.x, a.c * xp.y - a.s * ex.y);
+            x[1][j] = make_double2(a.s * xp.x + a.c * ex.x, a.s * xp.y + a.c * ex.y);
+          }
+          const double2 em = make_double2(b.eph.x, -b.eph.y);
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {  // columns: new_p = c x_p - s e^{-i phi} x_q, new_q = s x_p + c e^{-i phi} x_q
+            const double2 ex = cmul(em, x[i][1]), xp = x[i][0];
+            x[i][0] = make_double2(b.c * xp.x - b.s * ex.x, b.c * xp.y - b.s * ex.y);
+            x[i][1] = make_double2(b.s * xp.x + b.c * ex.x, b.s * xp.y + b.c * ex.y);
+          }
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+              if (rows[i] >= 0 && cols[j] >= 0) AE(rows[i], cols[j]) = x[i][j];
+        } else {
+          const int f = e - nh * nh, row = f % NB;
+          const JacPair b = pr[f / NB];
+          if (b.q >= 0) {
+            const double2 xp = VE(row, b.p), ex = cmul(make_double2(b.eph.x, -b.eph.y), VE(row, b.q));
+            VE(row, b.p) = make_double2(b.c * xp.x - b.s * ex.x, b.c * xp.y - b.s * ex.y);
+            VE(row, b.q) = make_double2(b.s * xp.x + b.c * ex.x, b.s * xp.y + b.c * ex.y);
           }
         }
       }
       __syncthreads();
-      // rows: A <- J^H A  (rows p,q of every column)
-      for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
-        const int p = e % NB, col = e / NB;
-        const int q = partner[p];
-        if (q < 0 || p > q) continue;
-        const double c = cs[p], s = sn[p];
-        const double2 eph = make_double2(ph_c[p], ph_s[p]);  // e^{i phi}
-        const double2 ap = AE(p, col), aq = AE(q, col);
-        // new_p = c ap - s e^{i phi} aq ; new_q = s ap + c e^{i phi} aq
-        const double2 ea = cmul(eph, aq);
-        AE(p, col) = make_double2(c * ap.x - s * ea.x, c * ap.y - s * ea.y);
-        AE(q, col) = make_double2(s * ap.x + c * ea.x, s * ap.y + c * ea.y);
-      }
-      __syncthreads();
-      // columns: A <- A J, V <- V J  (columns p,q of every row)
-      for (int e = threadIdx.x; e < 2 * NB * NB; e += blockDim.x) {
-        const int which = e / (NB * NB), rem = e % (NB * NB);
-        const int p = rem / NB, row = rem % NB;
-        const int q = partner[p];
-        if (q < 0 || p > q) continue;
-        const double c = cs[p], s = sn[p];
-        const double2 emph = make_double2(ph_c[p], -ph_s[p]);  // e^{-i phi}
-        double2* M = which ? V : A;
-        const double2 xp = M[(size_t)p * NB + row], xq = M[(size_t)q * NB + row];
-        // new_p = c xp - s e^{-i phi} xq ; new_q = s xp + c e^{-i phi} xq
-        const double2 ex = cmul(emph, xq);
-        M[(size_t)p * NB + row] = make_double2(c * xp.x - s * ex.x, c * xp.y - s * ex.y);
-        M[(size_t)q * NB + row] = make_double2(s * xp.x + c * ex.x, s * xp.y + c * ex.y);
-      }
-      __syncthreads();
     }
   }
-  if (threadIdx.x == 0) sweeps[k] = sweep;
+  if (t == 0) sweeps[k] = sweep;
   // eigenvalues = diag, sorted ascending with the eigenvector columns (like zheev)
   double* wk = w + (size_t)k * NB;
-  for (int i = threadIdx.x; i < NB; i += blockDim.x) cs[i] = AE(i, i).x;
+  for (int i = t; i < NB; i += nt) ev[i] = AE(i, i).x;
   __syncthreads();
-  for (int i = threadIdx.x; i < NB; i += blockDim.x) {
-    int rank = 0;
-    for (int j2 = 0; j2 < NB; ++j2) rank += (cs[j2] < cs[i]) || (cs[j2] == cs[i] && j2 < i);
-    partner[i] = rank;
-    wk[rank] = cs[i];
+  for (int i = t; i < NB; i += nt) {
+    int r = 0;
+    for (int j2 = 0; j2 < NB; ++j2) r += (ev[j2] < ev[i]) || (ev[j2] == ev[i] && j2 < i);
+    rank[i] = r;
+    wk[r] = ev[i];
   }
   __syncthreads();
   // permuted eigenvectors into A (A is no longer needed)
-  for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
+  for (int e = t; e < NB * NB; e += nt) {
     const int row = e % NB, col = e / NB;
-    AE(row, partner[col]) = VE(row, col);
+    Ag[(size_t)rank[col] * NB + row] = VE(row, col);
   }
 #undef AE
 #undef VE
 }
 
 cudaError_t launch_jacobi(const System& s, double2* A, double2* V, int max_sweeps, double* w, int* sweeps) {
-  const size_t smem = (size_t)s.NB * (4 * sizeof(double) + sizeof(int));
-  k_jacobi_herm<<<s.nkl, 1024, smem, s.launch_stream()>>>(A, V, s.NB, max_sweeps, w, sweeps);
-  return cudaGetLastError();
-}
-
-// ------------------------------------------------------------- rotation ---
-// out[k][n][i] = sum_m in[k][m][i] Z[k][n][m]   (zutmp(:,ib1) = sum_ib2 zu(:,ib2) za(ib2,ib1), diag.f90:120-126)
-constexpr int ROT_NB = 8;
-__global__ void __launch_bounds__(256) k_rotate(const double2* __restrict__ in, const double2* __restrict__ Z,
-                                                int NB, int NL, double2* __restrict__ out) {
-  const int k = blockIdx.y;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const double2* ink = in + (size_t)k * NB * NL;
-  const double2* Zk = Z + (size_t)k * NB * NB;
-  double2* outk = out + (size_t)k * NB * NL;
-  if (i >= NL) return;
-  for (int n0 = 0; n0 < NB; n0 += ROT_NB) {
-    double2 acc[ROT_NB];
-#pragma unroll
-    for (int t = 0; t < ROT_NB; ++t) acc[t] = make_double2(0, 0);
-    for (int m = 0; m < NB; ++m) {
-      const double2 x = ink[(size_t)m * NL + i];
-#pragma unroll
-      for (int t = 0; t < ROT_NB; ++t)
-        if (n0 + t < NB) acc[t] = cfma(x, __ldg(Zk + (size_t)(n0 + t) * NB + m), acc[t]);
-    }
-#pragma unroll
-    for (int t = 0; t < ROT_NB; ++t)
-      if (n0 + t < NB) outk[(size_t)(n0 + t) * NL + i] = acc[t];
+  const size_t base = jac_pair_bytes(s.NB) + 16, both = 2 * (size_t)s.NB * s.NB * sizeof(double2);
+  const int in_smem = base + both <= JAC_SMEM;
+  const size_t smem = base + (in_smem ? both : 0);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = raise_smem_limit((const void*)k_jacobi_herm, smem);
+    if (e != cudaSuccess) return e;
   }
-}
-
-cudaError_t launch_rotate(const System& s, const double2* in, const double2* Z, double2* out) {
-  dim3 grid((s.NL + 255) / 256, s.nkl);
-  k_rotate<<<grid, 256, 0, s.launch_stream()>>>(in, Z, s.NB, s.NL, out);
+  k_jacobi_herm<<<s.nkl, 1024, smem, s.launch_stream()>>>(A, V, s.NB, max_sweeps, in_smem, w, sweeps);
   return cudaGetLastError();
 }
 

@@ -527,7 +527,7 @@ int sgpu_destroy(sgpu_handle h) {
                   s->U, s->Up, s->Uw, s->red, s->stage, s->cur_part, s->nab12};
   for (void* p : bufs) cudaFree(p);
   void* gbufs[] = {s->gs_zu, s->gs_aux, s->gs_W, s->gs_st, s->gs_part, s->gs_A, s->gs_V, s->gs_w, s->gs_sweeps,
-                   s->occ_gs, s->gs_out, s->gs_res, s->gs_tb, s->vpsl, s->rho_d, s->exc_d, s->sp_blk,
+                   s->occ_gs, s->gs_out, s->gs_R, s->gs_bad, s->gs_M, s->gs_MR, s->gs_dots, s->gs_iters, s->gs_res, s->gs_tb, s->vpsl, s->rho_d, s->exc_d, s->sp_blk,
                    s->vloc_hist};
   for (void* p : gbufs) cudaFree(p);
   if (s->gs_h) cudaFreeHost(s->gs_h);
@@ -845,17 +845,24 @@ namespace {
 int gs_alloc(System* s) {
   if (s->gs_zu) return 0;
   const size_t nbl = (size_t)s->nkl * s->NB * s->NL;
-  const int nt = (s->NB + 15) / 16;
-  // split K so that the subspace GEMM has at least ~4 CTAs per SM
-  s->gs_nsplit = std::max(1, std::min(64, (4 * 148 + s->nkl * nt * nt - 1) / std::max(1, s->nkl * nt * nt)));
+  // partial products of the split-K kernels: about four 32 x 32 tiles per SM
+  const size_t nt = (s->NB + 31) / 32, nn = (size_t)s->nkl * s->NB * s->NB;
+  s->gs_part_elems = std::max<size_t>(nn * std::max<size_t>(1, std::min<size_t>(64, (4 * s->nsm) / (s->nkl * nt * nt))),
+                                      nn + (size_t)4 * s->nsm * 1024);
   CK(cudaMalloc(&s->gs_zu, nbl * sizeof(double2)));
   CK(cudaMalloc(&s->gs_aux, nbl * sizeof(double2)));
   CK(cudaMalloc(&s->gs_W, (size_t)sgpu::cg_work_vectors() * s->nkl * s->NL * sizeof(double2)));
   CK(cudaMalloc(&s->gs_st, s->nkl * sgpu::cg_state_bytes()));
-  CK(cudaMalloc(&s->gs_part, (size_t)s->gs_nsplit * s->nkl * s->NB * s->NB * sizeof(double2)));
+  CK(cudaMalloc(&s->gs_part, s->gs_part_elems * sizeof(double2)));
   CK(cudaMalloc(&s->gs_A, (size_t)s->nkl * s->NB * s->NB * sizeof(double2)));
   CK(cudaMalloc(&s->gs_V, (size_t)s->nkl * s->NB * s->NB * sizeof(double2)));
   CK(cudaMalloc(&s->gs_w, (size_t)s->nkl * s->NB * sizeof(double)));
+  CK(cudaMalloc(&s->gs_R, (size_t)s->nkl * 32 * 32 * sizeof(double2)));
+  CK(cudaMalloc(&s->gs_bad, (size_t)s->nkl * sizeof(int)));
+  CK(cudaMalloc(&s->gs_M, (size_t)s->nkl * s->NB * 256 * sizeof(double2)));
+  CK(cudaMalloc(&s->gs_MR, (size_t)s->nkl * s->NB * 256 * sizeof(double)));
+  CK(cudaMalloc(&s->gs_dots, (size_t)s->nkl * sgpu::CG_DOT_SPLITS * 256 * sizeof(double2)));
+  CK(cudaMalloc(&s->gs_iters, (size_t)s->nkl * s->NB * sizeof(int)));
   CK(cudaMalloc(&s->gs_sweeps, (size_t)s->nkl * sizeof(int)));
   CK(cudaMalloc(&s->gs_out, (size_t)s->nkl * s->NB * sizeof(double)));
   CK(cudaMalloc(&s->gs_res, (size_t)s->nkl * s->NB * sizeof(double)));
@@ -965,40 +972,37 @@ int sgpu_cg(sgpu_handle h, int ncg, double* esp_var, int* iters) {
   if (rc) return rc;
   const size_t NL = s->NL, nk = s->nkl;
   double2* W = s->gs_W;
-  auto vec = [&](int which) { return W + (size_t)which * nk * NL; };
-  std::vector<int> it_all(iters ? (size_t)s->nkl * s->NB : 0);
-  std::vector<char> st_h(s->nkl * sgpu::cg_state_bytes());
+  double2* zu = s->gs_zu;
+  auto vec = [&](int which) { return W + (size_t)which * nk * NL; };  // xk hxk txk gk pk pko htpsi ttpsi hk
+  const bool wide = sgpu::cg_wide(*s), proj = !wide, pre = s->cg_precond != 0;
+  // the gradient's projections and what follows them up to the direction pko
+  auto direction = [&](int ib, int iter) -> int {
+    if (wide) CK(sgpu::launch_cg_project(*s, zu, ib, 3, pre));
+    if (pre) {
+      CK(sgpu::launch_tpa(*s, vec(8), s->nkl, s->gs_tb, 1));                      // kinetic-energy factor
+      if (s->cg_precond == 2) CK(sgpu::launch_precond_net(*s, vec(8), s->nkl));  // learned refinement
+      if (wide) CK(sgpu::launch_cg_project(*s, zu, ib, 8, false));
+    }
+    if (wide || pre) CK(sgpu::launch_cg_dir(*s, zu, ib, iter, proj, pre));
+    return 0;
+  };
   for (int ib = 0; ib < s->NB; ++ib) {
-    CK(sgpu::launch_cg_begin(*s, s->gs_zu, W, s->gs_st, ib));
-    if ((rc = gs_hpsi(s, vec(0), vec(1), vec(2), s->nkl, 1))) return rc;   // xk -> hxk, txk
-    CK(sgpu::launch_cg_dot0(*s, W, s->gs_st));
+    if (wide) CK(sgpu::launch_cg_project(*s, zu, ib, -1, false));
+    CK(sgpu::launch_cg_open(*s, zu, ib, proj));
+    if ((rc = gs_hpsi(s, vec(0), vec(1), vec(2), s->nkl, 1))) return rc;     // xk -> hxk, txk
+    CK(sgpu::launch_cg_first(*s, zu, ib, proj, pre));
     for (int iter = 1; iter <= ncg; ++iter) {
-      if (s->cg_precond == 0) {  // the reference's CG (CG.f90:85-106)
-        CK(sgpu::launch_cg_pre(*s, s->gs_zu, W, s->gs_st, ib, iter));
-      } else {                   // preconditioned direction
-        CK(sgpu::launch_cg_grad(*s, s->gs_zu, W, s->gs_st, s->gs_tb, ib));
-        CK(sgpu::launch_tpa(*s, vec(8), s->nkl, s->gs_tb, 1));                      // kinetic-energy factor
-        if (s->cg_precond == 2) CK(sgpu::launch_precond_net(*s, vec(8), s->nkl));  // learned refinement
-        CK(sgpu::launch_cg_dir(*s, s->gs_zu, W, s->gs_st, ib, iter));
-      }
-      if ((rc = gs_hpsi(s, vec(5), vec(6), vec(7), s->nkl, 1))) return rc; // pko -> htpsi, ttpsi
-      CK(sgpu::launch_cg_post(*s, W, s->gs_st, iter));
+      if ((rc = direction(ib, iter))) return rc;
+      if ((rc = gs_hpsi(s, vec(5), vec(6), vec(7), s->nkl, 1))) return rc;  // pko -> htpsi, ttpsi
+      CK(sgpu::launch_cg_step(*s, zu, ib, iter, iter == ncg, proj, pre));
     }
-    CK(sgpu::launch_cg_end(*s, s->gs_zu, W, ib));
-    if ((rc = gs_hpsi(s, vec(0), vec(6), nullptr, s->nkl, 1))) return rc;  // H u_ib
-    CK(sgpu::launch_cg_resid(*s, W, s->occ_gs, s->gs_out, s->gs_res, ib));
-    if (iters) {
-      CK(cudaMemcpyAsync(st_h.data(), s->gs_st, st_h.size(), cudaMemcpyDeviceToHost, s->stream));
-      CK(cudaStreamSynchronize(s->stream));
-      for (int k = 0; k < s->nkl; ++k) {
-        int v;
-        std::memcpy(&v, st_h.data() + k * sgpu::cg_state_bytes() + 2 * sizeof(double) + sizeof(int), sizeof(int));
-        it_all[(size_t)k * s->NB + ib] = v;
-      }
-    }
+    if (wide) CK(sgpu::launch_cg_row(*s, zu, ib));
+    if ((rc = gs_hpsi(s, vec(0), vec(6), nullptr, s->nkl, 1))) return rc;    // H u_ib, for the residual
   }
+  CK(sgpu::launch_cg_open(*s, zu, s->NB, proj));  // the last band's residual
   if ((rc = gs_copy_out(s, s->gs_out, esp_var))) return rc;
-  if (iters) std::memcpy(iters, it_all.data(), it_all.size() * sizeof(int));
+  if (iters)
+    CK(cudaMemcpyAsync(iters, s->gs_iters, (size_t)s->nkl * s->NB * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));
   return 0;
 }
@@ -1091,7 +1095,7 @@ int sgpu_subspace_diag(sgpu_handle h, double* esp) {
   int rc = gs_ready(s, "sgpu_subspace_diag");
   if (rc) return rc;
   if ((rc = gs_hpsi(s, s->gs_zu, s->gs_aux, nullptr, s->nkl * s->NB, s->NB))) return rc;
-  CK(sgpu::launch_subspace_h(*s, s->gs_zu, s->gs_aux, s->gs_part, s->gs_nsplit, s->gs_A));
+  CK(sgpu::launch_subspace_h(*s, s->gs_zu, s->gs_aux, s->gs_part, s->gs_A));
   CK(sgpu::launch_jacobi(*s, s->gs_A, s->gs_V, 30, s->gs_w, s->gs_sweeps));
   CK(sgpu::launch_rotate(*s, s->gs_zu, s->gs_A, s->gs_aux));
   std::swap(s->gs_zu, s->gs_aux);

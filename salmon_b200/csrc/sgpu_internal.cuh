@@ -183,7 +183,14 @@ struct System {
   double2* gs_aux = nullptr;       // [nkl][NB][NL]  H zu_GS, rotation output
   double2* gs_W = nullptr;         // [8][nkl][NL]   CG work vectors
   void* gs_st = nullptr;           // [nkl] CG state
-  double2* gs_part = nullptr;      // [nsplit][nkl][NB][NB]
+  double2* gs_part = nullptr;      // [gs_part_elems] partial products of the split-K kernels
+  size_t gs_part_elems = 0;
+  double2* gs_R = nullptr;         // [nkl][32][32] inverse Cholesky factor of a Gram-Schmidt panel
+  int* gs_bad = nullptr;           // [nkl] panels left to the one-by-one Gram-Schmidt
+  double2* gs_M = nullptr;         // [nkl][NB][256] rows of (I + L)^-1, L the lower bands' overlaps (k_gs.cu)
+  double* gs_MR = nullptr;         // [nkl][NB][256] the same for the overlaps' real parts
+  double2* gs_dots = nullptr;      // [nkl][CG_DOT_SPLITS][256] partial inner products with the lower bands
+  int* gs_iters = nullptr;         // [nkl][NB] CG iterations of each band
   double2* gs_A = nullptr;         // [nkl][NB][NB]
   double2* gs_V = nullptr;         // [nkl][NB][NB]
   double* gs_w = nullptr;          // [nkl][NB]
@@ -191,7 +198,6 @@ struct System {
   double* occ_gs = nullptr;        // [nkl][NB]
   double* gs_out = nullptr;        // [nkl][NB] device results
   double* gs_h = nullptr;          // pinned host staging [nkl][NB]
-  int gs_nsplit = 0;
   bool have_gs = false;
   size_t U_rows = 0;               // orbitals U can hold
 
@@ -317,14 +323,20 @@ cudaError_t launch_energy(System& s, double* e_dev);
 
 // ground state (k_gs.cu)
 cudaError_t launch_gram_schmidt(const System& s, double2* zu);
-cudaError_t launch_cg_begin(const System& s, double2* zu, double2* W, void* st, int ib);
-cudaError_t launch_cg_dot0(const System& s, double2* W, void* st);
-cudaError_t launch_cg_pre(const System& s, const double2* zu, double2* W, void* st, int ib, int iter);
-cudaError_t launch_cg_post(const System& s, double2* W, void* st, int iter);
-cudaError_t launch_cg_end(const System& s, double2* zu, double2* W, int ib);
-cudaError_t launch_cg_resid(const System& s, double2* W, const double* occ_gs, double* esp_var, double* res, int ib);
-cudaError_t launch_cg_grad(const System& s, const double2* zu, double2* W, void* st, double* tband, int ib);
-cudaError_t launch_cg_dir(const System& s, const double2* zu, double2* W, void* st, int ib, int iter);
+// (launch_gram_schmidt: k_zgemm.cu; _panel: the one-by-one form for the bands p0 .. p0+pb-1
+// of the k-points with bad[k])
+cudaError_t launch_gram_schmidt_panel(const System& s, double2* zu, int p0, int pb, const int* bad);
+// CG of band ib (work vectors s.gs_W, see sgpu_cg): proj: the projections on the lower
+// bands run inside the kernels (cluster form); otherwise launch_cg_project and
+// launch_cg_row do them (cg_wide).  pre: with a preconditioner.
+constexpr int CG_DOT_SPLITS = 16;
+bool cg_wide(const System& s);
+cudaError_t launch_cg_open(const System& s, double2* zu, int ib, bool proj);
+cudaError_t launch_cg_first(const System& s, double2* zu, int ib, bool proj, bool pre);
+cudaError_t launch_cg_dir(const System& s, double2* zu, int ib, int iter, bool proj, bool pre);
+cudaError_t launch_cg_step(const System& s, double2* zu, int ib, int iter, bool last, bool proj, bool pre);
+cudaError_t launch_cg_project(const System& s, double2* zu, int ib, int which, bool copy_hk);
+cudaError_t launch_cg_row(const System& s, double2* zu, int ib);
 // Batched 3D FFT (sign -1 forward, +1 backward; normalise divides by NL) of
 // nvec grid functions, and the TPA preconditioner applied in place to nvec
 // vectors (vector v belongs to k-point v / vecs_per_k; tband_dev[v] its band's
@@ -344,8 +356,7 @@ cudaError_t launch_tpa(const System& s, double2* data, int nvec, const double* t
                        const int* kidx_dev = nullptr);
 size_t cg_state_bytes();
 int cg_work_vectors();
-cudaError_t launch_subspace_h(const System& s, const double2* U, const double2* HU, double2* part, int nsplit,
-                              double2* za);
+cudaError_t launch_subspace_h(const System& s, const double2* U, const double2* HU, double2* part, double2* za);
 cudaError_t launch_jacobi(const System& s, double2* A, double2* V, int max_sweeps, double* w, int* sweeps);
 cudaError_t launch_rotate(const System& s, const double2* in, const double2* Z, double2* out);
 

@@ -1,0 +1,96 @@
+"""The blocked forms of the ground-state routines at the sizes where they change shape:
+32-band panels of the Gram-Schmidt, 256-band blocks and the whole-GPU form of CG's
+projections, the shared- and global-memory eigensolver.
+
+Tolerances: FP64 sums of N terms in another order differ by a few eps times the
+condition of what they feed: 1e-12 for well-conditioned Gram-Schmidt, eps * kappa for
+a nearly dependent band, 1e-9 for CG (a few iterations amplify the rounding)."""
+import numpy as np
+import pytest
+
+from _helpers import rel
+from oracle import oracle as O
+from salmon_b200 import system as S
+
+pytestmark = pytest.mark.gpu
+
+
+def raw_system(grid, nk, nb, seed=5):
+    sysm, kAc, vloc, _ = S.small_system(*grid, nk=nk, nb=nb, seed=seed)
+    rng = np.random.default_rng(seed + 1)
+    z = rng.standard_normal((nk, nb, sysm.NL)) + 1j * rng.standard_normal((nk, nb, sysm.NL))
+    return sysm, kAc, vloc, z
+
+
+def handle(sysm, kAc, vloc, z):
+    from salmon_b200.rt import GpuSystem
+    g = GpuSystem(sysm)
+    g.set_vloc(vloc)
+    g.update_projector(kAc)
+    g.gs_set_state(z)
+    return g
+
+
+def gram_schmidt(sysm, kAc, vloc, z):
+    with handle(sysm, kAc, vloc, z) as g:
+        g.gram_schmidt()
+        return g.gs_get_state()
+
+
+@pytest.mark.parametrize("nb", [1, 31, 32, 33, 70])
+def test_gram_schmidt_panels(cuda_lib, nb):
+    case = raw_system((7, 9, 11), 2, nb)
+    out = gram_schmidt(*case)
+    assert rel(out, O.gram_schmidt(case[0], case[3])) < 1e-12
+
+
+def test_gram_schmidt_dependent_and_zero_bands(cuda_lib):
+    sysm, kAc, vloc, z = raw_system((7, 9, 11), 3, 40)
+    z[0, 5] = z[0, 3] + 1e-7 * z[0, 5]      # refused by the Cholesky of the first panel
+    z[1, 36] = z[1, 34] + 1e-7 * z[1, 36]   # of the second
+    ref = O.gram_schmidt(sysm, z)
+    out = gram_schmidt(sysm, kAc, vloc, z)
+    # kappa ~ 1e7: the dependent band itself moves by eps * kappa ~ 2e-9, and later ones with it
+    assert rel(out, ref) < 1e-7
+    assert rel(out[2], ref[2]) < 1e-12
+    ov = np.einsum("kbi,kci->kbc", out.conj(), out) * sysm.Hxyz
+    assert np.abs(ov - np.eye(40)).max() < 1e-7
+    z[2, 4] = 0.0                           # NaN from there on, as one by one
+    with np.errstate(all="ignore"):
+        ref = O.gram_schmidt(sysm, z)
+    out = gram_schmidt(sysm, kAc, vloc, z)
+    np.testing.assert_array_equal(np.isnan(out[2]).any(axis=1), np.isnan(ref[2]).any(axis=1))
+    assert rel(out[2, :4], ref[2, :4]) < 1e-12
+
+
+@pytest.mark.parametrize("grid,nk,nb,orthonormal", [
+    ((7, 9, 11), 2, 9, False),      # bands not orthogonal: the order of the projections counts
+    ((8, 8, 8), 1, 260, True),      # two blocks of lower bands
+    ((16, 16, 16), 1, 128, True),   # one k-point: projections over the whole GPU
+    ((16, 16, 16), 1, 128, False),
+])
+def test_cg_projections(cuda_lib, grid, nk, nb, orthonormal):
+    sysm, kAc, vloc, z = raw_system(grid, nk, nb)
+    z = S.orthonormalise(z, sysm.Hxyz) if orthonormal else z / np.sqrt((np.abs(z) ** 2).sum(-1, keepdims=True) * sysm.Hxyz)
+    with handle(sysm, kAc, vloc, z) as g:
+        esp, its = g.cg(2)
+        out = g.gs_get_state()
+    ref, esp_ref, its_ref = O.cg(sysm, kAc, vloc, z, 2)
+    np.testing.assert_array_equal(its, its_ref)
+    assert rel(out, ref) < 1e-9
+    assert rel(esp, esp_ref) < 1e-9
+
+
+@pytest.mark.parametrize("nb", [7, 82, 84, 128])  # A and V in shared memory up to 82 bands
+def test_subspace_diag_sizes(cuda_lib, nb):
+    sysm, kAc, vloc, z = raw_system((8, 9, 10), 2, nb)
+    z = S.orthonormalise(z, sysm.Hxyz)
+    with handle(sysm, kAc, vloc, z) as g:
+        esp = g.subspace_diag()
+        out = g.gs_get_state()
+    _, esp_ref = O.diag(sysm, kAc, vloc, z)
+    assert rel(esp, esp_ref) < 1e-11
+    ov = np.einsum("kbi,kci->kbc", out.conj(), out) * sysm.Hxyz
+    assert np.abs(ov - np.eye(nb)).max() < 1e-11
+    for k in range(2):
+        assert rel(out[k].T @ out[k].conj(), z[k].T @ z[k].conj()) < 1e-10
