@@ -19,19 +19,24 @@ constexpr int RHO_CHUNK = 64;
 
 template <typename R>
 __global__ void k_rho_partial(const C2<R>* __restrict__ zu, const double* __restrict__ occ_o, int norb, int NL,
-                              double* __restrict__ part) {
+                              int chunk, double* __restrict__ part) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= NL) return;
-  const int o0 = blockIdx.y * RHO_CHUNK;
-  const int o1 = min(o0 + RHO_CHUNK, norb);
+  const int o0 = blockIdx.y * chunk;
+  const int o1 = min(o0 + chunk, norb);
   double acc = 0.0;
   int o = o0;
-  for (; o + 4 <= o1; o += 4) {
-    double2 z[4];
+  // 16 loads in flight: on small grids (few CTAs) the chunk is a chain of load latencies
+  constexpr int UN = 16;
+  for (; o + UN <= o1; o += UN) {
+    C2<R> z[UN];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) z[u] = to_d2(zu[(size_t)(o + u) * NL + i]);
+    for (int u = 0; u < UN; ++u) z[u] = zu[(size_t)(o + u) * NL + i];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) acc += occ_o[o + u] * (z[u].x * z[u].x + z[u].y * z[u].y);
+    for (int u = 0; u < UN; ++u) {
+      const double2 v = to_d2(z[u]);
+      acc += occ_o[o + u] * (v.x * v.x + v.y * v.y);
+    }
   }
   for (; o < o1; ++o) {
     const double2 z = to_d2(zu[(size_t)o * NL + i]);
@@ -44,18 +49,25 @@ __global__ void k_rho_final(const double* __restrict__ part, int nchunk, int NL,
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= NL) return;
   double acc = 0.0;
+#pragma unroll 16
   for (int c = 0; c < nchunk; ++c) acc += part[(size_t)c * NL + i];
   rho[i] = acc;
 }
 
 cudaError_t launch_psi_rho(System& s, double* rho_dev) {
-  const int nchunk = (s.norb + RHO_CHUNK - 1) / RHO_CHUNK;
+  // chunks of 64 orbitals, of 16 (one round of loads) where those leave SMs without two CTAs
+  // and the partial densities fit
+  const int nblk = (s.NL + 255) / 256;
+  int chunk = RHO_CHUNK;
+  if (nblk * ((s.norb + RHO_CHUNK - 1) / RHO_CHUNK) < 2 * s.nsm && (size_t)((s.norb + 15) / 16) * s.NL <= s.red_elems)
+    chunk = 16;
+  const int nchunk = (s.norb + chunk - 1) / chunk;
   if ((size_t)nchunk * s.NL > s.red_elems) return cudaErrorInvalidValue;
-  dim3 grid((s.NL + 255) / 256, nchunk);
+  dim3 grid(nblk, nchunk);
   if (s.prec == SGPU_PREC_C64)
-    k_rho_partial<float><<<grid, 256, 0, s.launch_stream()>>>((const float2*)s.zu, s.occ_o, s.norb, s.NL, s.red);
+    k_rho_partial<float><<<grid, 256, 0, s.launch_stream()>>>((const float2*)s.zu, s.occ_o, s.norb, s.NL, chunk, s.red);
   else
-    k_rho_partial<double><<<grid, 256, 0, s.launch_stream()>>>((const double2*)s.zu, s.occ_o, s.norb, s.NL, s.red);
+    k_rho_partial<double><<<grid, 256, 0, s.launch_stream()>>>((const double2*)s.zu, s.occ_o, s.norb, s.NL, chunk, s.red);
   k_rho_final<<<(s.NL + 255) / 256, 256, 0, s.launch_stream()>>>(s.red, nchunk, s.NL, rho_dev);
   return cudaGetLastError();
 }

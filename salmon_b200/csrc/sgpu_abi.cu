@@ -88,6 +88,14 @@ int one_orbital_k(const System* s, int ik) { return (ik - s->NK_s) * s->NBocc; }
 // points, then the stencil pass (which may export its output to S).
 cudaError_t apply_h(System* s, int mode, sgpu::PassIO io, int o_beg, int nb, int nbk, int prec, bool u_from_S) {
   cudaError_t e;
+  if (sgpu::hpsi_point_wins(*s, nb, prec)) {  // small batches: point-parallel, W from the projections on the fly
+    if (s->nsp > 0) {
+      e = u_from_S ? sgpu::launch_uvpsi_from_S(*s, s->Sbuf, o_beg, nb, nbk, true)
+                   : sgpu::launch_uvpsi(*s, io.in, o_beg, nb, nbk, true, prec);
+      if (e != cudaSuccess) return e;
+    }
+    return sgpu::launch_hpsi_point(*s, mode, io, o_beg, nb, nbk, prec);
+  }
   if (s->nsp > 0) {
     if ((e = sgpu::launch_kb_term(*s, io.in, u_from_S, o_beg, nb, nbk, s->Wbuf, prec)) != cudaSuccess) return e;
     io.W = s->Wbuf;
@@ -910,7 +918,7 @@ int gs_hpsi(System* s, const double2* in, double2* out, double2* tt, int nb, int
   io.out = out;
   io.tt = tt;
   const int keep = s->nslab;
-  if (s->nyblk == 1) s->nslab = std::max(1, std::min(s->nsm / std::max(1, nb), s->NLx / 8));
+  if (s->nyblk == 1 && !sgpu::hpsi_point_wins(*s, nb, SGPU_PREC_C128)) s->nslab = std::max(1, std::min(s->nsm / std::max(1, nb), s->NLx / 8));
   const cudaError_t e = apply_h(s, tt ? 1 : 0, io, 0, nb, nbk, SGPU_PREC_C128, false);
   s->nslab = keep;
   CK(e);
@@ -1013,7 +1021,10 @@ int sgpu_set_vpsl(sgpu_handle h, const double* vpsl) {
   if (!s->vpsl) {
     CK(cudaMalloc(&s->vpsl, (size_t)s->NL * sizeof(double)));
     CK(cudaMalloc(&s->rho_d, (size_t)s->NL * sizeof(double)));
-    CK(cudaMalloc(&s->exc_d, 2 * sizeof(double)));
+    CK(cudaMalloc(&s->exc_d, (2 + 2 * sgpu::XC_PARTS + 1) * sizeof(double)));  // energies, partial energies, counter
+    s->xc_part = s->exc_d + 2;
+    s->xc_count = (unsigned*)(s->xc_part + 2 * sgpu::XC_PARTS);
+    CK(cudaMemsetAsync(s->xc_count, 0, sizeof(unsigned), s->stream));
   }
   CK(cudaMemcpyAsync(s->vpsl, vpsl, (size_t)s->NL * sizeof(double), cudaMemcpyHostToDevice, s->stream));
   CK(cudaStreamSynchronize(s->stream));
@@ -1280,6 +1291,7 @@ extern "C" int sgpu_autotune_step(sgpu_handle h, double dt, int reps, int* param
   cudaError_t err = cudaSuccess;
   std::vector<std::array<int, 6>> cands;
   if (sgpu::resident_step_fits(*s)) cands.push_back({2, old[1], old[2], old[3], old[4], old[5]});
+  cands.push_back({0, 1, 1, 1, 0, old[5]});  // the library's own choice (small grids: the point-parallel form)
   for (int pf : {1, 0})
     for (int pt : {1, 0})
       for (int ns : {1, 2, 4}) {

@@ -244,6 +244,8 @@ struct System {
   double* vpsl = nullptr;          // [NL] local pseudopotential (for the self-consistent Vloc)
   double* rho_d = nullptr;         // [NL] density used by the last potential update
   double* exc_d = nullptr;         // [2] Hartree and exchange-correlation energies
+  double* xc_part = nullptr;       // [2 x XC_PARTS] partial energies of the potential kernel's CTAs
+  unsigned* xc_count = nullptr;    // CTAs of the potential kernel that have written their energies (0 between launches)
   double* gs_res = nullptr;        // [nkl][NB] residual norms of the last sgpu_cg
   double* vloc_hist = nullptr;     // [2][NL] the etrs potential history Vloc_old(:,1:2) (allocated on first use)
 };
@@ -286,6 +288,11 @@ struct PassIO {
 void taylor_stage_coefs(double dt, double c[4][2]);
 // prec = -1 uses the handle's precision; SGPU_PREC_C128 forces FP64 (ground state).
 cudaError_t launch_hpsi_pass(const System& s, int mode, const PassIO& io, int o_beg, int nb, int nbk, int prec = -1);
+// The same application for a small batch, one thread per point (k_point.cu), with the
+// KB term taken from the projections in s.U instead of io.W; whether that form is the
+// faster one for nb orbitals.
+bool hpsi_point_wins(const System& s, int nb, int prec = -1);
+cudaError_t launch_hpsi_point(const System& s, int mode, const PassIO& io, int o_beg, int nb, int nbk, int prec = -1);
 // threads per CTA of the pass kernel for an NLy x NLz plane
 // Sets the shared-memory attribute of every stencil-pass kernel the handle can
 // launch (needed before capturing its launches into a graph).
@@ -352,6 +359,17 @@ void net_free(System& s);
 // (Vloc <- 3 Vloc - 3 hist1 + hist2, history shifted) on the device.
 cudaError_t launch_vloc_history(const System& s, bool extrapolate);
 cudaError_t launch_fft3d(const System& s, double2* data, int nvec, int sign, bool normalise);
+// The two parts of a transform pair around a factor in reciprocal space, three launches in
+// all: planes (z and y) forward, from complex data in place or from a real array; x forward,
+// the factor, x backward (fft_mid_poisson: 4 pi / |G|^2 / NL); planes backward with an
+// epilogue.  fft_fused_ok: the planes fit in shared memory.
+constexpr int XC_PARTS = 148;  // >= the largest axis and the CTAs of k_vloc
+cudaError_t launch_vloc(const System& s, const double2* z, const double* rho, double* part, double* energies_dev);
+bool fft_fused_ok(const System& s);
+cudaError_t launch_fft_planes_real(const System& s, const double* rho, double2* z);
+cudaError_t launch_fft_mid_poisson(const System& s, double2* z);
+cudaError_t launch_fft_planes_vloc(const System& s, const double2* z, const double* rho, double* part,
+                                   double* energies_dev);
 cudaError_t launch_tpa(const System& s, double2* data, int nvec, const double* tband_dev, int vecs_per_k,
                        const int* kidx_dev = nullptr);
 size_t cg_state_bytes();

@@ -1,0 +1,66 @@
+"""The forms for small batches and grids against the general ones and the oracle: the
+point-parallel H application (rows of odd length, grids below the stencil's width, points
+in several spheres), the fused transforms of the potential (every radix, one axis of
+length 1, planes beyond shared memory) and the density with few orbitals.
+
+Tolerances: complex(8) 1e-12 (FP64 sums in another order); complex(4) 2e-6, the bound of
+the complex(4) step against the FP64 oracle."""
+import numpy as np
+import pytest
+
+from _helpers import grid_system, rel
+from oracle import oracle as O, scf_oracle as X
+from salmon_b200 import system as S
+
+pytestmark = pytest.mark.gpu
+TOL = {"c128": 1e-12, "c64": 2e-6}
+
+
+@pytest.mark.parametrize("precision", ["c128", "c64"])
+@pytest.mark.parametrize("shape,nat,rps", [((8, 10, 12), 2, 1.6), ((3, 5, 7), 1, 0.9), ((9, 7, 11), 6, 3.0)])
+def test_point_form(cuda_lib, precision, shape, nat, rps):
+    from salmon_b200.rt import GpuSystem
+    sysm, kAc, vloc, zu = S.small_system(*shape, nk=2, nb=3, nat=nat, Rps=rps, seed=11)
+    _, zproj = O.update_projector(sysm, kAc)
+    z_in = zu if precision == "c128" else zu.astype(np.complex64).astype(np.complex128)
+    ref = O.hamiltonian(sysm, kAc, vloc, zproj, 0.01, z_in)
+    h_ref, tt_ref = O.hpsi(sysm, kAc, vloc, zproj, 2, z_in[1, 1], want_tt=True)
+    out = {}
+    for kernel in (0, 1):  # 0: small batches take the point form; 1: the stencil passes
+        with GpuSystem(sysm, precision) as g:
+            g.set_param("taylor_kernel", kernel)
+            g.set_state(zu)
+            g.set_vloc(vloc)
+            g.update_projector(kAc)
+            g.hamiltonian(0.01)
+            assert rel(g.get_state(), ref) < TOL[precision]
+            g.hamiltonian(0.01)  # projects from the sphere values that the first step exported
+            out[kernel] = g.get_state()
+            h, tt = g.hpsi_omp_KB_GS(2, z_in[1, 1])
+            assert rel(h, h_ref) < TOL[precision] and rel(tt, tt_ref) < TOL[precision]
+    assert rel(out[0], out[1]) < TOL[precision]
+
+
+@pytest.mark.parametrize("shape", [(8, 9, 12), (1, 6, 8), (16, 2, 27), (6, 81, 64), (4, 96, 96)])
+def test_fused_potential(cuda_lib, shape):
+    from salmon_b200.rt import GpuSystem
+    sysm = grid_system(shape)
+    rng = np.random.default_rng(3)
+    rho = rng.uniform(0.0, 0.5, sysm.NL)
+    vpsl = rng.standard_normal(sysm.NL)
+    v_ref, e_ref = X.vloc(rho, vpsl, shape, sysm.aL, sysm.Hxyz)
+    with GpuSystem(sysm) as g:
+        g.set_vpsl(vpsl)
+        for _ in range(2):  # the energies' counter is back at zero
+            e = g.update_vloc(rho)
+            assert rel(g.get_vloc(), v_ref) < 1e-12
+            assert rel(e, e_ref) < 1e-12
+
+
+@pytest.mark.parametrize("nk,nb", [(1, 1), (1, 15), (1, 17), (3, 33)])
+def test_density_chunks(cuda_lib, nk, nb):
+    from salmon_b200.rt import GpuSystem
+    sysm, _, _, zu = S.small_system(5, 6, 7, nk=nk, nb=nb)
+    with GpuSystem(sysm) as g:
+        g.set_state(zu)
+        assert rel(g.psi_rho_RT(), O.psi_rho(sysm, zu)) < 1e-12
