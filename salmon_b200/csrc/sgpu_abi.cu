@@ -450,19 +450,30 @@ int sgpu_create(const sgpu_desc* d, int precision, sgpu_handle* out) {
   UP(s->kbq, kbq);
   UP(s->kb_multi, kb_multi);
   UP(s->lqi, lqi);
-  {  // sp_blk: first sphere point of every (plane, y-block) and the plane end
-    const int nb1 = s->nyblk + 1;
-    std::vector<int> cnt((size_t)s->NLx * s->nyblk, 0), blk((size_t)s->NLx * nb1, 0);
-    for (int r : qrow) cnt[(size_t)(r / s->NLy) * s->nyblk + (r % s->NLy) / s->NYB]++;
-    int acc = 0;
-    for (int x = 0; x < s->NLx; ++x) {
-      for (int yb = 0; yb < s->nyblk; ++yb) {
-        blk[(size_t)x * nb1 + yb] = acc;
-        acc += cnt[(size_t)x * s->nyblk + yb];
+  {  // first sphere point of every (plane, block of `rows` rows) and the plane end
+    auto blocks = [&](int nblk, int rows, int* most) {
+      const int nb1 = nblk + 1;
+      std::vector<int> cnt((size_t)s->NLx * nblk, 0), blk((size_t)s->NLx * nb1, 0);
+      for (int r : qrow) cnt[(size_t)(r / s->NLy) * nblk + (r % s->NLy) / rows]++;
+      int acc = 0;
+      for (int x = 0; x < s->NLx; ++x) {
+        for (int yb = 0; yb < nblk; ++yb) {
+          blk[(size_t)x * nb1 + yb] = acc;
+          acc += cnt[(size_t)x * nblk + yb];
+          if (most) *most = std::max(*most, cnt[(size_t)x * nblk + yb]);
+        }
+        blk[(size_t)x * nb1 + nblk] = acc;
       }
-      blk[(size_t)x * nb1 + s->nyblk] = acc;
-    }
+      return blk;
+    };
+    const std::vector<int> blk = blocks(s->nyblk, s->NYB, nullptr);
     UP(s->sp_blk, blk);
+    for (int pr = 0; pr < 2; ++pr) {
+      const int rows = s->p2_rows[pr] = sgpu::pass2_rows(pr, s->NLy, s->NLz);
+      if (rows == 0) continue;
+      const std::vector<int> blk2 = blocks(s->NLy / rows, rows, &s->p2_maxpts[pr]);
+      UP(s->p2_blk[pr], blk2);
+    }
   }
   UP(s->occ_o, occo);
 #undef UP
@@ -535,7 +546,7 @@ int sgpu_destroy(sgpu_handle h) {
                   s->U, s->Up, s->Uw, s->red, s->stage, s->cur_part, s->nab12};
   for (void* p : bufs) cudaFree(p);
   void* gbufs[] = {s->gs_zu, s->gs_aux, s->gs_W, s->gs_st, s->gs_part, s->gs_A, s->gs_V, s->gs_w, s->gs_sweeps,
-                   s->occ_gs, s->gs_out, s->gs_R, s->gs_bad, s->gs_M, s->gs_MR, s->gs_dots, s->gs_iters, s->gs_res, s->gs_tb, s->vpsl, s->rho_d, s->exc_d, s->sp_blk,
+                   s->occ_gs, s->p2_blk[0], s->p2_blk[1], s->gs_out, s->gs_R, s->gs_bad, s->gs_M, s->gs_MR, s->gs_dots, s->gs_iters, s->gs_res, s->gs_tb, s->vpsl, s->rho_d, s->exc_d, s->sp_blk,
                    s->vloc_hist};
   for (void* p : gbufs) cudaFree(p);
   if (s->gs_h) cudaFreeHost(s->gs_h);
@@ -1296,9 +1307,9 @@ extern "C" int sgpu_autotune_step(sgpu_handle h, double dt, int reps, int* param
     for (int pt : {1, 0})
       for (int ns : {1, 2, 4}) {
         if (ns > 1 && s->NLx / ns < 8) continue;
-        for (int sp : {-1, 0, 1, 2, 4, 8}) {  // -1: the split tile, 0: the band-group tile kernel
-          if (sp <= 0 && !sgpu::kb_tile_fits(*s)) continue;
-          cands.push_back({1, pf, pt, ns, sp < 0 ? 3 : (sp ? 2 : 1), sp > 0 ? sp : old[5]});
+        for (int sp : {-2, -1, 0, 1, 2, 4, 8}) {  // -2: the library's choice, -1: the split tile, 0: the tile kernel
+          if ((sp == -1 || sp == 0) && !sgpu::kb_tile_fits(*s)) continue;
+          cands.push_back({1, pf, pt, ns, sp == -2 ? 0 : (sp < 0 ? 3 : (sp ? 2 : 1)), sp > 0 ? sp : old[5]});
         }
       }
   for (const auto& c : cands) {

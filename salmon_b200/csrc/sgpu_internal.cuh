@@ -204,6 +204,10 @@ struct System {
   // tuning
   int nslab = 1;                   // x-slabs per orbital in the stencil pass
   int nyblk = 1, NYB = 0;          // y-blocks per plane (planes wider than 512 threads) and their rows
+  // two-row pass, by precision: rows of a block (0: no such form), its most sphere points,
+  // [NLx*(NLy/rows+1)] the first sphere point of each (plane, block)
+  int p2_rows[2] = {0, 0}, p2_maxpts[2] = {0, 0};
+  int* p2_blk[2] = {nullptr, nullptr};
   int* sp_blk = nullptr;           // [NLx*(nyblk+1)] first sphere point of each (plane, y-block)
   int pass_tab = 1;                // stencil pass: Vloc/sphere-index tables through the ring (two-point form)
   int pass_fixed = 1;              // stencil pass: compile-time plane shapes with a 9-plane ring (complex(4))
@@ -293,6 +297,7 @@ cudaError_t launch_hpsi_pass(const System& s, int mode, const PassIO& io, int o_
 // faster one for nb orbitals.
 bool hpsi_point_wins(const System& s, int nb, int prec = -1);
 cudaError_t launch_hpsi_point(const System& s, int mode, const PassIO& io, int o_beg, int nb, int nbk, int prec = -1);
+int pass2_rows(int prec, int NLy, int NLz);
 // threads per CTA of the pass kernel for an NLy x NLz plane
 // Sets the shared-memory attribute of every stencil-pass kernel the handle can
 // launch (needed before capturing its launches into a graph).

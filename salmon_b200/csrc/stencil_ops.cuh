@@ -95,6 +95,20 @@ __device__ __forceinline__ void stencil_pair(double2& v, double2& wa, double2 p,
   wa.x = fma(cn, p.x - m.x, wa.x);
   wa.y = fma(cn, p.y - m.y, wa.y);
 }
+// the first pair of a sum: v = cl (p + m) (FV), wa = cn (p - m) (FW), no zeroed accumulator
+template <bool FV, bool FW>
+__device__ __forceinline__ void stencil_pair_first(float2& v, float2& wa, float2 p, float2 m, float2 cl, float2 cn) {
+  const float2 sum = __fadd2_rn(p, m);
+  const float2 dif = __ffma2_rn(m, make_float2(-1.f, -1.f), p);
+  v = FV ? __fmul2_rn(cl, sum) : __ffma2_rn(cl, sum, v);
+  wa = FW ? __fmul2_rn(cn, dif) : __ffma2_rn(cn, dif, wa);
+}
+template <bool FV, bool FW>
+__device__ __forceinline__ void stencil_pair_first(double2& v, double2& wa, double2 p, double2 m, double cl, double cn) {
+  const double2 sum = make_double2(p.x + m.x, p.y + m.y), dif = make_double2(p.x - m.x, p.y - m.y);
+  v = FV ? make_double2(cl * sum.x, cl * sum.y) : make_double2(fma(cl, sum.x, v.x), fma(cl, sum.y, v.y));
+  wa = FW ? make_double2(cn * dif.x, cn * dif.y) : make_double2(fma(cn, dif.x, wa.x), fma(cn, dif.y, wa.y));
+}
 template <typename R> __device__ __forceinline__ auto kpair(double k) {
   if constexpr (std::is_same<R, float>::value) return make_float2((float)k, (float)k); else return k;
 }
