@@ -332,11 +332,13 @@ enum {
   SGPU_PARAM_KB_KERNEL = 5,   /* KB term of H psi: 1 band-group tile kernel (32 bands of a k-point per
                                  CTA, pipelined gathers), 2 band-quad kernel (UVPSI_SPLIT warps per
                                  4 bands), 3 the tile kernel's projections over KB_SPLIT point ranges
-                                 then a point-parallel field kernel, 0 the tile kernel for
-                                 complex(4) when its grid has >= 2 CTAs per SM, else form 3          */
-  SGPU_PARAM_PASS_FIXED = 6,  /* stencil pass, complex(4): 1 uses the compile-time plane shapes
-                                 (16x16, 16x32, 20x20, 32x32 planes, 48x48 in three y-blocks: 9-plane
-                                 ring, constant offsets) where they fit, 0 the generic kernel         */
+                                 then a point-parallel field kernel, 0 the library's choice: atoms
+                                 of few points staged whole, else the tile kernel for complex(4)
+                                 when its grid has >= 2 CTAs per SM, else form 3                      */
+  SGPU_PARAM_PASS_FIXED = 6,  /* stencil pass: 1 uses the compile-time plane shapes where they fit
+                                 (two rows per thread on 16x32, 32x32, 48x48 and, complex(8), 16x16
+                                 planes; complex(4) 16x16 and 20x20 with constant offsets), 0 the
+                                 generic kernel                                                       */
   SGPU_PARAM_CUR_FIXED = 7,   /* current and energy stencils on 32x32 and 48x48 planes: 1 the
                                  current's march with two rows per thread (32x32 split over two CTAs,
                                  48x48 over six) and the energy's over four / six CTAs, 2 the

@@ -749,6 +749,169 @@ static cudaError_t launch_kb_split_t(const System& s, const void* in, int ld_in,
   return cudaGetLastError();
 }
 
+// ------------------------------------------------------------ KB atom ---
+// The KB term for atoms whose points fit in shared memory whole (at most KBA_PTS: the
+// usual spacings of 0.5 bohr and more): one CTA per (32 bands of a k-point, projector item).
+// The streamed forms above run 123 points in four chunks, each with a wait and a barrier, and
+// read the projectors twice; their time there is the fill of two pipelines.  Here every
+// value of the CTA is requested at once (each warp gathers four bands, the point indices in
+// its registers), one barrier later each warp holds its band quad's projections in
+// registers, exchanges them by shuffles and writes its part of W, without another barrier.
+// Bound by the fetch latency that several CTAs per SM overlap, and by HBM.  Measured times:
+// see launch_kb_term.
+constexpr int KBA_PTS = 256;
+template <typename R>
+struct KbaGeom {
+  static size_t srow(int mps) { return (size_t)(mps + 15) / 16 * 16 + 4; }  // band rows: 4 rows x 4 points in distinct banks
+  static size_t zrow(int mps) { return (size_t)(mps + 15) / 16 * 16 + 2; }
+  static size_t smem(int mps) {
+    return sizeof(C2<R>) * KBT_BANDS * srow(mps) + sizeof(double2) * 4 * zrow(mps) + sizeof(int) * KBA_PTS;
+  }
+};
+
+template <typename R>
+__global__ void __launch_bounds__(256) k_kb_atom(const C2<R>* __restrict__ in, int ld_in, int o_beg, int nb, int nbk,
+                                                 int kl0, int ngrp, const double2* __restrict__ zproj, int Nlma, int Nps,
+                                                 const int* __restrict__ idx, const int* __restrict__ kbq,
+                                                 const int* __restrict__ atom_off, const int4* __restrict__ items,
+                                                 const int* __restrict__ lma_list, const int* __restrict__ iuV,
+                                                 double scale, double2* __restrict__ U, int nsp, C2<R>* __restrict__ W,
+                                                 int SROW, int ZROW) {
+  using T = C2<R>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* Sb = reinterpret_cast<T*>(smem_raw);                        // [32][SROW]
+  double2* Zb = reinterpret_cast<double2*>(Sb + KBT_BANDS * SROW);  // [4][ZROW]
+  int* kqs = reinterpret_cast<int*>(Zb + 4 * ZROW);              // [KBA_PTS] W index (-1: multi)
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int kq = blockIdx.x / ngrp, grp = blockIdx.x - kq * ngrp;
+  const int kl = kl0 + kq;
+  const int o_lo = max(o_beg, kl * nbk + grp * KBT_BANDS);
+  const int o_hi = min(min(o_beg + nb, (kl + 1) * nbk), kl * nbk + (grp + 1) * KBT_BANDS);
+  if (o_lo >= o_hi) return;  // whole CTA leaves together
+  const int nbq = o_hi - o_lo;
+  const int4 item = items[blockIdx.y];
+  const int a = item.x, l0 = item.y, np = item.z;
+  const int p0 = atom_off[a], mps = atom_off[a + 1] - p0;
+  const int mpr = (mps + 15) / 16 * 16;
+  int ix[KBA_PTS / 32];
+#pragma unroll
+  for (int i = 0; i < KBA_PTS / 32; ++i) {
+    const int j = lane + 32 * i;
+    ix[i] = j < mps ? __ldg(idx + p0 + j) : -1;
+  }
+#pragma unroll
+  for (int b = warp; b < KBT_BANDS; b += 8) {
+    if (b >= nbq) break;
+    const T* src = in + (size_t)(o_lo + b - o_beg) * ld_in;
+    T* dst = Sb + b * SROW + lane;
+#pragma unroll
+    for (int i = 0; i < KBA_PTS / 32; ++i) {
+      if (32 * i + lane >= mpr) break;
+      if (ix[i] >= 0) { if constexpr (sizeof(T) == 8) cp_async8(dst + 32 * i, src + ix[i]); else cp_async16(dst + 32 * i, src + ix[i]); }
+      else dst[32 * i] = mk<R>(0, 0);
+    }
+  }
+  {  // projector rows: two warps a row; sphere indices
+    const int p = warp & 3;
+    const double2* zs = p < np ? zproj + ((size_t)kl * Nlma + lma_list[l0 + p]) * Nps : nullptr;
+    for (int j = lane + 32 * (warp >> 2); j < mpr; j += 64) {
+      if (zs && j < mps) cp_async16(Zb + p * ZROW + j, zs + j);
+      else Zb[p * ZROW + j] = make_double2(0.0, 0.0);
+    }
+    if (t < mps) cp_async4(kqs + t, kbq + p0 + t);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  if (4 * warp >= nbq) return;  // no CTA-wide barrier follows
+
+  // ---- the warp's 8x8 tile of projections, four accumulator chains
+  const int krow = lane & 3, n = lane >> 2;
+  double c[4][2] = {};
+  {
+    const T* sb = Sb + (4 * warp + (n >> 1)) * SROW + krow;               // B column n: band n/2 of the quad, Re/Im
+    const double* za = reinterpret_cast<const double*>(Zb + (n & 3) * ZROW + krow) + (n >> 2);  // A row n
+    for (int j = 0; j < mpr; j += 16)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const T v = sb[j + 4 * u];
+        mma_f64_8x8x4(c[u][0], c[u][1], za[2 * (j + 4 * u)], (double)((n & 1) ? v.y : v.x));
+      }
+  }
+  const double x0 = (c[0][0] + c[1][0]) + (c[2][0] + c[3][0]), x1 = (c[0][1] + c[1][1]) + (c[2][1] + c[3][1]);
+  // lanes 0-15 hold rows p (Re zproj), lanes 16-31 rows p+4 (Im zproj) of band lane & 3
+  const double d0 = __shfl_down_sync(0xffffffffu, x0, 16);
+  const double d1 = __shfl_down_sync(0xffffffffu, x1, 16);
+  double2 u = make_double2(0.0, 0.0);
+  if (lane < 16) {
+    const int p = lane >> 2, o = o_lo + 4 * warp + (lane & 3);
+    if (p < np && o < o_hi) {
+      const int ilma = lma_list[l0 + p];
+      const double f = scale * (double)iuV[ilma];
+      u = make_double2((x0 + d1) * f, (x1 - d0) * f);
+      U[(size_t)(o - o_beg) * Nlma + ilma] = u;
+    }
+  }
+  // B fragment of the second product: projector krow, band n/2
+  const double ux = __shfl_sync(0xffffffffu, u.x, krow * 4 + (n >> 1));
+  const double uy = __shfl_sync(0xffffffffu, u.y, krow * 4 + (n >> 1));
+  const double bre = (n & 1) ? uy : ux;   // rows of Re zproj
+  const double bim = (n & 1) ? ux : -uy;  // rows of Im zproj
+  const int oc = o_lo + 4 * warp + krow;  // the orbital of this lane's C elements
+  const bool cvalid = oc < o_hi;
+  T* Wb = W + (size_t)(cvalid ? oc - o_beg : 0) * nsp;
+  const double2* zb = Zb + krow * ZROW + n;
+#pragma unroll 4
+  for (int j = 0; j < mps; j += 8) {
+    const double2 z = zb[j];
+    double w0 = 0.0, w1 = 0.0;
+    mma_f64_8x8x4(w0, w1, z.x, bre);
+    mma_f64_8x8x4(w0, w1, z.y, bim);
+    if (cvalid && j + n < mps) {
+      const int q = kqs[j + n];
+      if (q >= 0) Wb[q] = mk<R>((R)w0, (R)w1);
+    }
+  }
+}
+
+static bool kb_atom_fits(const System& s) { return s.max_mps >= 1 && s.max_mps <= KBA_PTS; }
+// Where the whole-atom form is the faster one: three CTAs' values fit an SM, and, in
+// complex(4), at most eight CTAs per SM (beyond, the streamed form's finer interleaving of
+// gathers and stores wins by 10%).  KB term, whole atom against the form taken otherwise, us:
+// complex(4) 16^3 x 1024 orbitals 10.4 / 16.4, 16x16x32 x 1024 16.5 / 18.6, 20^3 x 2048 26.8 /
+// 28.8, 48^3 x 100 23.7 / 26.8, x 1728 523 / 467 (not taken); complex(8) 8^3 x 1024 6.3 /
+// 16.5, 16^3 x 1024 14.5 / 22.7, 48^3 x 800 269 / 301, 20^3 x 2048 (251 points) 51 / 46 (not
+// taken).
+static bool kb_atom_wins(const System& s, bool f, int ctas) {
+  const size_t smem = f ? KbaGeom<float>::smem(s.max_mps) : KbaGeom<double>::smem(s.max_mps);
+  return kb_atom_fits(s) && 3 * smem <= 224 * 1024 && (!f || ctas <= 8 * s.nsm);
+}
+
+template <typename R>
+static cudaError_t launch_kb_atom_t(const System& s, const void* in, int ld_in, const int* idx, int o_beg, int nb,
+                                    int nbk, void* W) {
+  const int kl0 = o_beg / nbk, kl1 = (o_beg + nb - 1) / nbk;
+  const int ngrp = (nbk + KBT_BANDS - 1) / KBT_BANDS;
+  const size_t smem = KbaGeom<R>::smem(s.max_mps);
+  if (!s.kb_smem_ok) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(s.stream, &cs);
+    if (e != cudaSuccess) return e;
+    if (cs == cudaStreamCaptureStatusNone && (e = prepare_kb(s)) != cudaSuccess) return e;
+  }
+  dim3 grid((kl1 - kl0 + 1) * ngrp, s.nitems);
+  k_kb_atom<R><<<grid, 256, smem, s.launch_stream()>>>(
+      (const C2<R>*)in, ld_in, o_beg, nb, nbk, kl0, ngrp, s.zproj64, s.Nlma, s.Nps, idx, s.kbq, s.atom_off, s.items,
+      s.lma_list, s.iuV_d, s.Hxyz, s.U, s.nsp, (C2<R>*)W, (int)KbaGeom<R>::srow(s.max_mps),
+      (int)KbaGeom<R>::zrow(s.max_mps));
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess || s.n_multi == 0) return e;
+  dim3 g2((s.n_multi + 255) / 256, (nb + KU - 1) / KU);
+  k_kbfield_multi<R><<<g2, 256, 0, s.launch_stream()>>>(s.U, nb, o_beg, nbk, s.zproj64, s.Nlma, s.Nps, s.rec, s.cont,
+                                                         s.kb_multi, s.n_multi, s.nsp, (C2<R>*)W);
+  return cudaGetLastError();
+}
+
 static int kb_tile_ctas(const System& s, int o_beg, int nb, int nbk) {
   const int kl0 = o_beg / nbk, kl1 = (o_beg + nb - 1) / nbk;
   return (kl1 - kl0 + 1) * ((nbk + KBT_BANDS - 1) / KBT_BANDS) * s.nitems;
@@ -764,6 +927,10 @@ cudaError_t prepare_kb(const System& s) {
   if (e == cudaSuccess) e = raise_smem_limit((const void*)k_kb_tile<double>, KbtGeom<double>::smem(s.Nps));
   if (e == cudaSuccess) e = raise_smem_limit((const void*)k_kb_tile<float, true>, KbtGeom<float>::smem(s.Nps));
   if (e == cudaSuccess) e = raise_smem_limit((const void*)k_kb_tile<double, true>, KbtGeom<double>::smem(s.Nps));
+  if (kb_atom_fits(s)) {
+    if (e == cudaSuccess) e = raise_smem_limit((const void*)k_kb_atom<float>, KbaGeom<float>::smem(s.max_mps));
+    if (e == cudaSuccess) e = raise_smem_limit((const void*)k_kb_atom<double>, KbaGeom<double>::smem(s.max_mps));
+  }
   s.kb_smem_ok = e == cudaSuccess;
   return e;
 }
@@ -793,6 +960,9 @@ cudaError_t launch_kb_term(const System& s, const void* in, bool from_S, int o_b
   // 0.058 / 0.055 ms (band quad 0.079) and 0.089 / 0.087 ms.  The split projections
   // on the FP64 CUDA cores instead of the MMAs (lanes over points, 4 bands x 4
   // projectors a thread) were slower at every shape (0.163, 0.119, 0.086 ms complex(4)).
+  if (s.kb_kernel == 0 && kb_atom_wins(s, f, kb_tile_ctas(s, o_beg, nb, nbk)))
+    return f ? launch_kb_atom_t<float>(s, src, ld, idx, o_beg, nb, nbk, W)
+             : launch_kb_atom_t<double>(s, src, ld, idx, o_beg, nb, nbk, W);
   const bool fits = kb_tile_fits(s);
   const bool tile_first = f && kb_tile_ctas(s, o_beg, nb, nbk) >= 2 * s.nsm;
   if (fits && (s.kb_kernel == 3 || (s.kb_kernel == 0 && !tile_first)))
