@@ -339,11 +339,10 @@ enum {
                                  (two rows per thread on 16x32, 32x32, 48x48 and, complex(8), 16x16
                                  planes; complex(4) 16x16 and 20x20 with constant offsets), 0 the
                                  generic kernel                                                       */
-  SGPU_PARAM_CUR_FIXED = 7,   /* current and energy stencils on 32x32 and 48x48 planes: 1 the
-                                 current's march with two rows per thread (32x32 split over two CTAs,
-                                 48x48 over six) and the energy's over four / six CTAs, 2 the
-                                 current's march with one row per thread (four / six CTAs), 0 the
-                                 generic kernels                                                     */
+  SGPU_PARAM_CUR_FIXED = 7,   /* current stencil on 32x32 and 48x48 planes: 1 the march with two rows
+                                 per thread at compile-time shapes (32x32 split over two CTAs, 48x48
+                                 over six), 2 one row per thread (four / six CTAs), 0 the march for
+                                 any shape, which the energy always takes                            */
   SGPU_PARAM_TAYLOR_KERNEL = 8, /* Taylor step: 1 four stencil passes over all orbitals (any grid), 2
                                  the orbitals of a band group resident in one CTA's shared memory for
                                  the whole step (16x16, 16x32 and 20x20 planes where they fit), 0 the

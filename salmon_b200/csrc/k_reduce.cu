@@ -99,115 +99,195 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh /*[32*NV]*
 // sums F,G,H = 2 sum Im(conj(psi) sum_n nab_n psi(+n)) (stencil/F90/current.f90),
 // with forward neighbours only (n = 1..4), as the reference's stencil has them.
 //
-// One CTA of NT threads per orbital marches along x.  Thread t owns the plane
-// points t, t+NT, ... (P of them); for each it keeps psi at planes x..x+4 in a
-// register queue (converted to FP64 once, on load), so the x-neighbours cost
-// nothing; plane x is staged in FP64 in shared memory (double-buffered) for the
-// y and z neighbours.  Every element is read from HBM once (the four wrap planes
-// twice) and converted once; the loads run D planes ahead of their use.  Sums are FP64, per thread in plane order, then a
-// fixed-order block sum: out[o][4].
+// The orbital's planes are marched along x, the planes ahead in a register queue (FP64,
+// converted once on load), the current plane staged in FP64 in shared memory for the y and
+// z neighbours.  Sums are FP64, per thread in plane order, then a fixed-order block sum.
 struct Nab12 {
   double v[12];  // nabx(1:4), naby(1:4), nabz(1:4): kernel parameters, read from the parameter bank
 };
 
+// The march for any plane shape, two rows per thread: the plane is split into blocks of GB
+// rows (even; the last may be shorter), one CTA per (orbital, block); thread (r, z) owns the
+// points of rows 2r and 2r+1, so row 2r+1 is a y neighbour in registers and the four rows
+// after it are read once for both.  A CTA stages its rows and the four rows after them.
 //
-// GY, GZ (non-zero): the plane shape at compile time, so the neighbour offsets are
-// shifts and masks the compiler recomputes instead of holding them in registers;
-// MB: CTAs per SM the register budget is cut for.
-template <typename R, int NT, int P, int D, int GY = 0, int GZ = 0, int MB = 1>
-__global__ void __launch_bounds__(NT, MB) k_current_march(const C2<R>* __restrict__ zu, int NLx, int NLy_, int NLz_,
-                                                        const Nab12 nab, double* __restrict__ out) {
+// EKIN: the kinetic energy instead of the current.  Summed over the periodic grid, the
+// backward neighbours give the same products as the forward ones,
+//   sum_i conj(e_i) (e_{i+n} + e_{i-n}) = 2 sum_i Re(conj(e_i) e_{i+n}),
+//   sum_i conj(e_i) (e_{i+n} - e_{i-n}) = 2i sum_i Im(conj(e_i) e_{i+n}),
+// so tpsum = sum conj(e) (lap0_2 e - 0.5 v - i w) (stencil/F90/total_energy.f90:93-180) needs
+// the forward neighbours only: half of the arithmetic and of the shared-memory reads.  With
+// one CTA per plane and 24 neighbours through L1, 20^3 x 2048 orbitals, complex(8), took
+// 1.14 ms; now 0.17 (sgpu_energy_terms: see launch_energy).  The current with this form:
+// see current_stencil.
+// out[o][block][4] = {sum |e|^2, F/2, G/2, H/2}, or [o][block][2] = {Re tpsum, 0}.
+struct FwdCoef {
+  double lap0_2;    // EKIN: -(lapx(0)+lapy(0)+lapz(0))/2
+  double lap[12];   // EKIN: lapx(1:4), lapy(1:4), lapz(1:4)
+  double nab[12];   // nabx(1:4), naby(1:4), nabz(1:4)
+};
+
+template <typename R, bool EKIN>
+__global__ void __launch_bounds__(256, 2) k_fwd_march(const C2<R>* __restrict__ zu, int NLx, int NLy, int NLz, int GB,
+                                                      int nblk, int NBocc, const double* __restrict__ kAc,
+                                                      const FwdCoef c, double* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int NLy = GZ ? GY : NLy_, NLz = GZ ? GZ : NLz_;
-  const int NYZ = NLy * NLz;
-  double2* buf = reinterpret_cast<double2*>(smem_raw);  // [2][NYZ]
   __shared__ double sh[32 * 4];
-  const int o = blockIdx.x, t = threadIdx.x;
+  double2* buf = reinterpret_cast<double2*>(smem_raw);  // [2][(GB+4)*NLz]
+  const int RB = (GB + 4) * NLz;
+  const int o = blockIdx.x / nblk, h = blockIdx.x - o * nblk, t = threadIdx.x, nt = blockDim.x;
+  const int NYZ = NLy * NLz, rows = min(GB, NLy - h * GB);
   const C2<R>* E = zu + (size_t)o * NLx * NYZ;
-  const double* nb = nab.v;
-  int yr[P][4], zi[P][4], own[P];
-  bool ok[P];
+  const int y0 = 2 * (t / NLz), z = t - (t / NLz) * NLz;
+  const bool act = y0 < rows, two = y0 + 1 < rows;
+  const int own = act ? (h * GB + y0) * NLz + z : 0;
+  const int own_b = two ? own + NLz : own;
+  int zo[4];
 #pragma unroll
-  for (int p = 0; p < P; ++p) {
-    const int i = t + NT * p;
-    ok[p] = i < NYZ;
-    own[p] = ok[p] ? i : 0;
-    const int y = own[p] / NLz, z = own[p] - (own[p] / NLz) * NLz;
-#pragma unroll
-    for (int n = 1; n <= 4; ++n) {
-      int yn = y + n, zn = z + n;
-      while (yn >= NLy) yn -= NLy;
-      while (zn >= NLz) zn -= NLz;
-      yr[p][n - 1] = yn * NLz + z;
-      zi[p][n - 1] = y * NLz + zn;
-    }
+  for (int n = 1; n <= 4; ++n) {
+    int zz = z + n;
+    while (zz >= NLz) zz -= NLz;
+    zo[n - 1] = zz - z;
   }
-  double2 q[5][P];  // q[m][p]: plane x+m at point p
+  double k[3] = {0, 0, 0};
+  if (EKIN) {
+    const int kl = o / NBocc;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) k[d] = kAc[3 * kl + d];
+  }
+  auto load = [&](int x, int i, bool ok) -> double2 {
+    return ok ? to_d2(__ldg(E + (size_t)x * NYZ + i)) : make_double2(0, 0);
+  };
+  // register queues: at phase P (plane x = 5i + P) plane x+m sits in slot (P+m) % 5
+  double2 qa[5], qb[5];
 #pragma unroll
   for (int m = 0; m < 5; ++m) {
-    const int xm = m < NLx ? m : m % NLx;
-#pragma unroll
-    for (int p = 0; p < P; ++p) q[m][p] = ok[p] ? to_d2(__ldg(E + (size_t)xm * NYZ + own[p])) : make_double2(0, 0);
+    const int xm = m % NLx;
+    qa[m] = load(xm, own, act);
+    qb[m] = load(xm, own_b, two);
   }
-  C2<R> nxt[D][P];  // planes x+5 .. x+4+D in flight
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    const int xm = (5 + d) % NLx;
-#pragma unroll
-    for (int p = 0; p < P; ++p) nxt[d][p] = ok[p] ? __ldg(E + (size_t)xm * NYZ + own[p]) : C2<R>{};
-  }
-  // a plane's bytes (bulk L2 prefetch needs 16-byte multiples; 0: no prefetch)
-  const unsigned pf_bytes = ((size_t)NYZ * sizeof(C2<R>)) % 16 == 0 ? (unsigned)(NYZ * sizeof(C2<R>)) : 0u;
-  double v[4] = {0, 0, 0, 0};  // jt, F (x), G (y), H (z)
-  for (int x = 0; x < NLx; ++x) {
-    double2* pl = buf + (size_t)(x & 1) * NYZ;
-#pragma unroll
-    for (int p = 0; p < P; ++p)
-      if (ok[p]) pl[own[p]] = q[0][p];
-    if (t == 0 && pf_bytes) {  // plane x+5+D+4 into L2 for the load issued four steps from now
-      prefetch_l2_bulk(E + (size_t)((x + 9 + D) % NLx) * NYZ, pf_bytes);
+  int xn = 5 % NLx;
+  C2<R> na = __ldg(E + (size_t)xn * NYZ + own), nb = __ldg(E + (size_t)xn * NYZ + own_b);  // in flight
+  xn = xn + 1 < NLx ? xn + 1 : 0;
+  double v[4] = {0, 0, 0, 0};
+  int x = 0;
+  auto step = [&](auto phase) -> bool {
+    constexpr int P = decltype(phase)::value;
+    double2* pl = buf + (x & 1) * RB;
+    const double2 ea = qa[P % 5], eb = qb[P % 5];
+    double2* pa = pl + y0 * NLz + z;
+    if (act) pa[0] = ea;
+    if (two) pa[NLz] = eb;
+    for (int i = t; i < 4 * NLz; i += nt) {
+      int hr = h * GB + rows + i / NLz;
+      while (hr >= NLy) hr -= NLy;
+      pl[rows * NLz + i] = to_d2(__ldg(E + (size_t)x * NYZ + hr * NLz + i % NLz));
     }
     __syncthreads();
+    if (act) {
+      double2 r[5];  // rows y0 + 1 .. y0 + 5 at column z
+      r[0] = two ? eb : pa[NLz];
 #pragma unroll
-    for (int p = 0; p < P; ++p) {
-      if (!ok[p]) continue;
-      const double2 e = q[0][p];
-      v[0] += e.x * e.x + e.y * e.y;
-      double2 sx = make_double2(0, 0), sy = make_double2(0, 0), sz = make_double2(0, 0);
+      for (int m = 1; m < 4; ++m) r[m] = pa[(m + 1) * NLz];
+      r[4] = two ? pa[5 * NLz] : make_double2(0, 0);
+      const double2 zero = make_double2(0, 0);
+      if constexpr (EKIN) {
+        double2 la = zero, lb = zero, ta = zero, tb = zero;  // sum lap e(+n), sum k nab e(+n)
 #pragma unroll
-      for (int n = 1; n <= 4; ++n) {
-        const double2 ex = q[n][p];
-        const double2 ey = pl[yr[p][n - 1]];
-        const double2 ez = pl[zi[p][n - 1]];
-        sx.x += nb[n - 1] * ex.x; sx.y += nb[n - 1] * ex.y;
-        sy.x += nb[3 + n] * ey.x; sy.y += nb[3 + n] * ey.y;
-        sz.x += nb[7 + n] * ez.x; sz.y += nb[7 + n] * ez.y;
+        for (int d = 0; d < 3; ++d) {
+          double2 wa = zero, wb = zero;
+#pragma unroll
+          for (int n = 1; n <= 4; ++n) {
+            const double2 fa = d == 0 ? qa[(P + n) % 5] : (d == 1 ? r[n - 1] : pa[zo[n - 1]]);
+            const double2 fb = d == 0 ? qb[(P + n) % 5] : (d == 1 ? r[n] : (two ? pa[NLz + zo[n - 1]] : zero));
+            const double cl = c.lap[4 * d + n - 1], cn = c.nab[4 * d + n - 1];
+            la.x = fma(cl, fa.x, la.x); la.y = fma(cl, fa.y, la.y);
+            lb.x = fma(cl, fb.x, lb.x); lb.y = fma(cl, fb.y, lb.y);
+            wa.x = fma(cn, fa.x, wa.x); wa.y = fma(cn, fa.y, wa.y);
+            wb.x = fma(cn, fb.x, wb.x); wb.y = fma(cn, fb.y, wb.y);
+          }
+          ta.x = fma(k[d], wa.x, ta.x); ta.y = fma(k[d], wa.y, ta.y);
+          tb.x = fma(k[d], wb.x, tb.x); tb.y = fma(k[d], wb.y, tb.y);
+        }
+        v[0] = fma(ea.x, ea.x, fma(ea.y, ea.y, fma(eb.x, eb.x, fma(eb.y, eb.y, v[0]))));
+        v[1] += fma(ea.x, la.x, ea.y * la.y) + fma(eb.x, lb.x, eb.y * lb.y);  // Re(conj(e) l)
+        v[2] += fma(ea.x, ta.y, -ea.y * ta.x) + fma(eb.x, tb.y, -eb.y * tb.x);  // Im(conj(e) t)
+      } else {
+        v[0] = fma(ea.x, ea.x, fma(ea.y, ea.y, fma(eb.x, eb.x, fma(eb.y, eb.y, v[0]))));
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          double2 wa = zero, wb = zero;
+#pragma unroll
+          for (int n = 1; n <= 4; ++n) {
+            const double2 fa = d == 0 ? qa[(P + n) % 5] : (d == 1 ? r[n - 1] : pa[zo[n - 1]]);
+            const double2 fb = d == 0 ? qb[(P + n) % 5] : (d == 1 ? r[n] : (two ? pa[NLz + zo[n - 1]] : zero));
+            const double cn = c.nab[4 * d + n - 1];
+            wa.x = fma(cn, fa.x, wa.x); wa.y = fma(cn, fa.y, wa.y);
+            wb.x = fma(cn, fb.x, wb.x); wb.y = fma(cn, fb.y, wb.y);
+          }
+          // aimag(conjg(e) s) = e.x s.y - e.y s.x, point a then point b
+          v[1 + d] = fma(eb.x, wb.y, fma(-eb.y, wb.x, fma(ea.x, wa.y, fma(-ea.y, wa.x, v[1 + d]))));
+        }
       }
-      // aimag(conj(e) * s) = e.x s.y - e.y s.x
-      v[1] += e.x * sx.y - e.y * sx.x;
-      v[2] += e.x * sy.y - e.y * sy.x;
-      v[3] += e.x * sz.y - e.y * sz.x;
     }
-    const int xl = (x + 5 + D) % NLx;  // the plane that enters the pipeline
-#pragma unroll
-    for (int p = 0; p < P; ++p) {
-      q[0][p] = q[1][p];
-      q[1][p] = q[2][p];
-      q[2][p] = q[3][p];
-      q[3][p] = q[4][p];
-      q[4][p] = ok[p] ? to_d2(nxt[0][p]) : make_double2(0, 0);
-#pragma unroll
-      for (int d = 0; d + 1 < D; ++d) nxt[d][p] = nxt[d + 1][p];
-      nxt[D - 1][p] = ok[p] ? __ldg(E + (size_t)xl * NYZ + own[p]) : C2<R>{};
-    }
+    qa[P % 5] = act ? to_d2(na) : make_double2(0, 0);  // plane x+5 takes the slot of plane x
+    qb[P % 5] = two ? to_d2(nb) : make_double2(0, 0);
+    na = __ldg(E + (size_t)xn * NYZ + own);
+    nb = __ldg(E + (size_t)xn * NYZ + own_b);
+    xn = xn + 1 < NLx ? xn + 1 : 0;
+    ++x;
+    return x < NLx;
+  };
+  for (;;) {
+    if (!step(std::integral_constant<int, 0>{})) break;
+    if (!step(std::integral_constant<int, 1>{})) break;
+    if (!step(std::integral_constant<int, 2>{})) break;
+    if (!step(std::integral_constant<int, 3>{})) break;
+    if (!step(std::integral_constant<int, 4>{})) break;
   }
   block_sum<4>(v, sh);
   if (t == 0) {
-    out[4 * (size_t)o] = v[0];
-    out[4 * (size_t)o + 1] = v[1];
-    out[4 * (size_t)o + 2] = v[2];
-    out[4 * (size_t)o + 3] = v[3];
+    if (EKIN) {
+      out[2 * (size_t)blockIdx.x] = c.lap0_2 * v[0] - v[1] + 2.0 * v[2];
+      out[2 * (size_t)blockIdx.x + 1] = 0.0;
+    } else {
+#pragma unroll
+      for (int m = 0; m < 4; ++m) out[4 * (size_t)blockIdx.x + m] = v[m];
+    }
   }
+}
+
+// rows of a block: the largest even number whose row pairs' points fit 256 threads, the
+// blocks of a plane as equal as that allows
+int march_rows(int NLy, int NLz) {
+  const int most = std::max(2, 2 * (256 / NLz)), nblk = (NLy + most - 1) / most;
+  return ((NLy + nblk - 1) / nblk + 1) / 2 * 2;
+}
+int march_blocks(int NLy, int NLz) {
+  const int GB = march_rows(NLy, NLz);
+  return (NLy + GB - 1) / GB;
+}
+
+template <typename R, bool EKIN>
+static cudaError_t fwd_march(System& s, double* out, int& nx) {
+  FwdCoef c;
+  c.lap0_2 = -(s.lap[0][0] + s.lap[1][0] + s.lap[2][0]) * 0.5;
+  for (int n = 0; n < 4; ++n)
+    for (int d = 0; d < 3; ++d) {
+      c.lap[4 * d + n] = s.lap[d][n + 1];
+      c.nab[4 * d + n] = s.nab[d][n + 1];
+    }
+  const int GB = march_rows(s.NLy, s.NLz);
+  nx = march_blocks(s.NLy, s.NLz);
+  const int nt = (GB / 2 * s.NLz + 31) / 32 * 32;
+  const size_t smem = 2 * (size_t)(GB + 4) * s.NLz * sizeof(double2);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = raise_smem_limit((const void*)k_fwd_march<R, EKIN>, smem);
+    if (e != cudaSuccess) return e;
+  }
+  k_fwd_march<R, EKIN><<<s.norb * nx, nt, smem, s.launch_stream()>>>((const C2<R>*)s.zu, s.NLx, s.NLy, s.NLz, GB, nx,
+                                                                     s.NBocc, s.kAc_d, c, out);
+  return cudaGetLastError();
 }
 
 // The x-march with each GY x GZ plane split over NP CTAs of GY/NP rows (one
@@ -384,68 +464,6 @@ static cudaError_t current_march_yh(System& s, const Nab12& nab, double* out) {
   k_current_march_yh<R, GY, GZ, NP><<<NP * s.norb, GY / NP * GZ, 0, s.launch_stream()>>>((const C2<R>*)s.zu, s.NLx,
                                                                                           nab, out);
   return cudaGetLastError();
-}
-
-// Planes of more than 1024 points: one CTA per (orbital, x-plane), the
-// neighbours read through L1/L2 (CTAs of one orbital are adjacent in launch
-// order, so the x-planes ahead are L2 hits); part[o][x][4].
-template <typename R>
-__global__ void __launch_bounds__(256, 2) k_current_plane(const C2<R>* __restrict__ zu, int NLx, int NLy, int NLz,
-                                                           const double* __restrict__ nab12, double* __restrict__ part) {
-  __shared__ double sh[32 * 4];
-  const int o = blockIdx.x / NLx, x = blockIdx.x - (blockIdx.x / NLx) * NLx;
-  const int NYZ = NLy * NLz;
-  const C2<R>* E = zu + (size_t)o * NLx * NYZ;
-  const C2<R>* P0 = E + (size_t)x * NYZ;
-  const C2<R>* Px[4];
-#pragma unroll
-  for (int n = 1; n <= 4; ++n) {
-    int xn = x + n;
-    while (xn >= NLx) xn -= NLx;
-    Px[n - 1] = E + (size_t)xn * NYZ;
-  }
-  double nb[12];
-#pragma unroll
-  for (int k = 0; k < 12; ++k) nb[k] = nab12[k];
-  double v[4] = {0, 0, 0, 0};
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int y = warp; y < NLy; y += nw) {
-    int yr[4];
-#pragma unroll
-    for (int n = 1; n <= 4; ++n) {
-      int yn = y + n;
-      while (yn >= NLy) yn -= NLy;
-      yr[n - 1] = yn * NLz;
-    }
-    for (int z = lane; z < NLz; z += 32) {
-      const int i = y * NLz + z;
-      const double2 e = to_d2(__ldg(P0 + i));
-      v[0] += e.x * e.x + e.y * e.y;
-      double2 sx = make_double2(0, 0), sy = make_double2(0, 0), sz = make_double2(0, 0);
-#pragma unroll
-      for (int n = 1; n <= 4; ++n) {
-        int zn = z + n;
-        while (zn >= NLz) zn -= NLz;
-        const double2 ex = to_d2(__ldg(Px[n - 1] + i));
-        const double2 ey = to_d2(__ldg(P0 + yr[n - 1] + z));
-        const double2 ez = to_d2(__ldg(P0 + y * NLz + zn));
-        sx.x += nb[n - 1] * ex.x; sx.y += nb[n - 1] * ex.y;
-        sy.x += nb[3 + n] * ey.x; sy.y += nb[3 + n] * ey.y;
-        sz.x += nb[7 + n] * ez.x; sz.y += nb[7 + n] * ez.y;
-      }
-      v[1] += e.x * sx.y - e.y * sx.x;
-      v[2] += e.x * sy.y - e.y * sy.x;
-      v[3] += e.x * sz.y - e.y * sz.x;
-    }
-  }
-  block_sum<4>(v, sh);
-  if (threadIdx.x == 0) {
-    double* d = part + ((size_t)o * NLx + x) * 4;
-    d[0] = v[0];
-    d[1] = v[1];
-    d[2] = v[2];
-    d[3] = v[3];
-  }
 }
 
 // Weighted projections for the nonlocal current (current.f90:247-265):
@@ -653,31 +671,12 @@ __global__ void k_current_sum(const double* __restrict__ jo, int norb, double* _
 }
 
 
-// scratch of launch_current (part [norb][NLx][4], jo [norb][3], 12 coefficients)
-// and of launch_energy (part [norb][NLx][2], eo [norb][2], 25 coefficients)
-size_t current_red_elems(int norb, int NLx) { return (size_t)norb * NLx * 4 + 3 * (size_t)norb + 32; }
+// scratch of launch_current (part [norb][rows][4], jo [norb][3]) and of launch_energy
+// (part [norb][rows][2], eo [norb][2])
+size_t current_red_elems(int norb, int rows) { return (size_t)norb * rows * 4 + 3 * (size_t)norb + 32; }
 
-template <typename R, int NT, int P, int D, int GY = 0, int GZ = 0, int MB = 1>
-static cudaError_t current_march(System& s, const Nab12& nab, double* out) {
-  const size_t smem = 2 * (size_t)s.NLy * s.NLz * sizeof(double2);
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(k_current_march<R, NT, P, D, GY, GZ, MB>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  k_current_march<R, NT, P, D, GY, GZ, MB><<<s.norb, NT, smem, s.launch_stream()>>>((const C2<R>*)s.zu, s.NLx, s.NLy,
-                                                                                    s.NLz, nab, out);
-  return cudaGetLastError();
-}
-
-// the x-marching form up to 1024 points per plane (one point per thread, up to
-// 1024 threads within 64 registers: the coefficients live in the parameter
-// bank), the plane-parallel form beyond.  Measured at 32^3 x 2048 orbitals
-// (complex(4)): 0.60 ms, against 0.61 ms with 512 threads x 2 points and 0.69 ms
-// with 256 x 4 (spills).
 template <typename R>
-static cudaError_t current_stencil(System& s, const Nab12& nab, const double* nab12, double* part, int& nx) {
-  const int NYZ = s.NLy * s.NLz;
+static cudaError_t current_stencil(System& s, const Nab12& nab, double* part, int& nx) {
   nx = 1;
   // 32x32 planes: two CTAs of 16 rows per orbital plane, two rows per thread at
   // three CTAs per SM (value 2: four CTAs of 8 rows, one row per thread).
@@ -699,27 +698,20 @@ static cudaError_t current_stencil(System& s, const Nab12& nab, const double* na
     nx = 6;
     return s.cur_fixed == 2 ? current_march_yh<R, 48, 48, 6>(s, nab, part) : current_march_y2<R, 48, 48, 6>(s, nab, part);
   }
-  if (NYZ <= 256) return current_march<R, 256, 1, 1>(s, nab, part);
-  if (NYZ <= 512) return current_march<R, 512, 1, 1>(s, nab, part);
-  if (NYZ <= 1024) return current_march<R, 1024, 1, 1>(s, nab, part);
-  nx = s.NLx;
-  k_current_plane<R><<<s.norb * s.NLx, 256, 0, s.launch_stream()>>>((const C2<R>*)s.zu, s.NLx, s.NLy, s.NLz, nab12,
-                                                                     part);
-  return cudaGetLastError();
+  // other planes: row blocks of any shape.  Whole planes per CTA (to 1024 points) and one CTA
+  // per plane beyond, in brackets, ms: 16x16x32 x 1024 orbitals, complex(4) 0.061 (0.088), 20^3 x
+  // 2048 0.143 (0.217), 8^3 x 1024 0.008 (0.021).  At 32^3 and 48^3 it is slower than the fixed
+  // forms above: 0.49 / 0.33 and, 800 orbitals, 0.75 / 0.52.
+  return fwd_march<R, false>(s, part, nx);
 }
 
 // The stencil sums {jt, F, G, H} of the resident orbitals into part[o][nx][4].
-// The 12 nab coefficients of the plane form live at the end of the handle's
-// reduction scratch.
 cudaError_t launch_current_stencil(System& s, double* part, int& nx) {
   Nab12 nab;
   for (int n = 0; n < 4; ++n)
     for (int d = 0; d < 3; ++d) nab.v[4 * d + n] = s.nab[d][n + 1];
   nx = 1;
-  // s.nab12 (device, set at creation) for the plane form; no scratch shared with
-  // work that may run beside this on the handle's other stream
-  return s.prec == SGPU_PREC_C64 ? current_stencil<float>(s, nab, s.nab12, part, nx)
-                                 : current_stencil<double>(s, nab, s.nab12, part, nx);
+  return s.prec == SGPU_PREC_C64 ? current_stencil<float>(s, nab, part, nx) : current_stencil<double>(s, nab, part, nx);
 }
 
 // The weighted projections of the nonlocal current, Uw[o][ilma][w]
@@ -753,9 +745,9 @@ cudaError_t launch_current_proj(System& s) {
 }
 
 cudaError_t launch_current(System& s, double* jav_dev) {
-  double* part = s.red;                              // [norb][nx][4]
-  double* jo = part + (size_t)s.norb * s.NLx * 4;    // [norb][3]
-  if ((size_t)s.norb * s.NLx * 4 + 3 * (size_t)s.norb + 12 > s.red_elems) return cudaErrorInvalidValue;
+  double* part = s.red;                              // [norb][nx][4], nx <= part_rows
+  double* jo = part + (size_t)s.norb * s.part_rows * 4;  // [norb][3]
+  if ((size_t)s.norb * s.part_rows * 4 + 3 * (size_t)s.norb + 12 > s.red_elems) return cudaErrorInvalidValue;
   int nx = 1;
   cudaError_t e;
   if (!s.cur_valid) {
@@ -778,150 +770,6 @@ cudaError_t launch_current(System& s, double* jav_dev) {
 }
 
 // -------------------------------------------------------------- energy ---
-// tpsum = sum conj(psi) (lap0_2 psi - 0.5 v - i w)  (stencil/F90/total_energy.f90:93-180)
-// One CTA per (orbital, x-plane), planes of an orbital adjacent in launch
-// order (the neighbour planes are L2 hits), laid out like k_current_plane; the plane's
-// two sums go to part[o][x][2] and are added in plane order by k_energy_comb.
-template <typename R>
-__global__ void __launch_bounds__(256, 2) k_ekin_plane(const C2<R>* __restrict__ zu, int NLx, int NLy, int NLz,
-                                                        int NBocc, const double* __restrict__ kAc,
-                                                        const double* __restrict__ coef, double* __restrict__ part) {
-  __shared__ double sh[32 * 2];
-  const int o = blockIdx.x / NLx, x = blockIdx.x - (blockIdx.x / NLx) * NLx, kl = o / NBocc;
-  const int NYZ = NLy * NLz;
-  const C2<R>* E = zu + (size_t)o * NLx * NYZ;
-  const C2<R>* P0 = E + (size_t)x * NYZ;
-  const C2<R>* Pp[4];
-  const C2<R>* Pm[4];
-#pragma unroll
-  for (int n = 1; n <= 4; ++n) {
-    int xp = x + n, xm = x - n;
-    while (xp >= NLx) xp -= NLx;
-    while (xm < 0) xm += NLx;
-    Pp[n - 1] = E + (size_t)xp * NYZ;
-    Pm[n - 1] = E + (size_t)xm * NYZ;
-  }
-  // coef: [0] = lap0_2, [1..12] = lapt, [13..24] = nab
-  const double A = coef[0];
-  double lapt[12], nabt[12];
-#pragma unroll
-  for (int n = 0; n < 12; ++n) {
-    lapt[n] = coef[1 + n];
-    nabt[n] = kAc[3 * kl + n / 4] * coef[13 + n];
-  }
-  double v2[2] = {0, 0};
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int y = warp; y < NLy; y += nw) {
-    int yp[4], ym[4];
-#pragma unroll
-    for (int n = 1; n <= 4; ++n) {
-      int a = y + n, b = y - n;
-      while (a >= NLy) a -= NLy;
-      while (b < 0) b += NLy;
-      yp[n - 1] = a * NLz;
-      ym[n - 1] = b * NLz;
-    }
-    for (int z = lane; z < NLz; z += 32) {
-      const int i = y * NLz + z;
-      const double2 e = to_d2(__ldg(P0 + i));
-      double2 v = make_double2(0, 0), w = make_double2(0, 0);
-#pragma unroll
-      for (int n = 1; n <= 4; ++n) {
-        int zp = z + n, zm = z - n;
-        while (zp >= NLz) zp -= NLz;
-        while (zm < 0) zm += NLz;
-        const double2 a1 = to_d2(__ldg(Pp[n - 1] + i)), a2 = to_d2(__ldg(Pm[n - 1] + i));
-        const double2 b1 = to_d2(__ldg(P0 + yp[n - 1] + z)), b2 = to_d2(__ldg(P0 + ym[n - 1] + z));
-        const double2 c1 = to_d2(__ldg(P0 + y * NLz + zp)), c2 = to_d2(__ldg(P0 + y * NLz + zm));
-        v.x += lapt[n - 1] * (a1.x + a2.x) + lapt[3 + n] * (b1.x + b2.x) + lapt[7 + n] * (c1.x + c2.x);
-        v.y += lapt[n - 1] * (a1.y + a2.y) + lapt[3 + n] * (b1.y + b2.y) + lapt[7 + n] * (c1.y + c2.y);
-        w.x += nabt[n - 1] * (a1.x - a2.x) + nabt[3 + n] * (b1.x - b2.x) + nabt[7 + n] * (c1.x - c2.x);
-        w.y += nabt[n - 1] * (a1.y - a2.y) + nabt[3 + n] * (b1.y - b2.y) + nabt[7 + n] * (c1.y - c2.y);
-      }
-      // z = A e - 0.5 v - i w ;  F += conj(e) z
-      const double2 zz = make_double2(A * e.x - 0.5 * v.x + w.y, A * e.y - 0.5 * v.y - w.x);
-      v2[0] += e.x * zz.x + e.y * zz.y;
-      v2[1] += e.x * zz.y - e.y * zz.x;
-    }
-  }
-  block_sum<2>(v2, sh);
-  if (threadIdx.x == 0) {
-    part[((size_t)o * NLx + x) * 2] = v2[0];
-    part[((size_t)o * NLx + x) * 2 + 1] = v2[1];
-  }
-}
-
-// The energy stencil as an x-march (GY x GZ planes split over NP CTAs of GY/NP
-// rows, one point per thread): psi at planes x-4..x+4 in a register queue
-// (FP64, converted once), plane x staged in FP64 in shared memory with four halo
-// rows on each side for the +-y neighbours.  The FD coefficients are kernel
-// parameters; k enters through nabt = k_d nab_d.  part[o][h][2].
-struct EkinCoef {
-  double lap0_2;     // -(lapx(0)+lapy(0)+lapz(0))/2
-  double lapt[12];   // lapx(1:4), lapy(1:4), lapz(1:4)
-  double nab[12];    // nabx(1:4), naby(1:4), nabz(1:4)
-};
-
-template <typename R, int GY, int GZ, int NP>
-__global__ void __launch_bounds__(GY / NP * GZ) k_ekin_march_yh(const C2<R>* __restrict__ zu, int NLx, int NBocc,
-                                                               const double* __restrict__ kAc, const EkinCoef c,
-                                                               double* __restrict__ out) {
-  constexpr int NYH = GY / NP, NT = NYH * GZ, NYZ = GY * GZ, RB = (NYH + 8) * GZ;
-  static_assert(NT % 32 == 0 && NT <= 1024 && 8 * GZ <= NT, "one point per thread, halos loaded by the first rows");
-  __shared__ double2 buf[2][RB];
-  __shared__ double sh[32 * 2];
-  const int o = blockIdx.x / NP, h = blockIdx.x - (blockIdx.x / NP) * NP, t = threadIdx.x;
-  const int kl = o / NBocc;
-  const C2<R>* E = zu + (size_t)o * NLx * NYZ;
-  double nabt[12];
-#pragma unroll
-  for (int n = 0; n < 12; ++n) nabt[n] = kAc[3 * kl + n / 4] * c.nab[n];
-  const int yl = t / GZ, z = t - (t / GZ) * GZ;
-  const int y0 = h * NYH;
-  const int own = (y0 + yl) * GZ + z;
-  // halo rows of threads t < 8 GZ: rows y0-4..y0-1 then y0+NYH..y0+NYH+3
-  const int hr = t / GZ;
-  const int hrow = hr < 4 ? (y0 - 4 + hr + GY) % GY : (y0 + NYH + hr - 4) % GY;
-  const int hdst = (hr < 4 ? hr : NYH + hr) * GZ + z;
-  const int hsrc = hrow * GZ + z;
-  double2 q[9];  // q[m]: plane x-4+m
-#pragma unroll
-  for (int m = 0; m < 9; ++m) q[m] = to_d2(__ldg(E + (size_t)((m - 4 + 4 * NLx) % NLx) * NYZ + own));
-  C2<R> nxt = __ldg(E + (size_t)(5 % NLx) * NYZ + own);
-  double v2[2] = {0, 0};
-  for (int x = 0; x < NLx; ++x) {
-    double2* pl = buf[x & 1];
-    pl[(4 + yl) * GZ + z] = q[4];
-    if (t < 8 * GZ) pl[hdst] = to_d2(__ldg(E + (size_t)x * NYZ + hsrc));
-    __syncthreads();
-    const double2 e = q[4];
-    double2 v = make_double2(0, 0), w = make_double2(0, 0);
-#pragma unroll
-    for (int n = 1; n <= 4; ++n) {
-      const double2 a1 = q[4 + n], a2 = q[4 - n];
-      const double2 b1 = pl[(4 + yl + n) * GZ + z], b2 = pl[(4 + yl - n) * GZ + z];
-      const double2 c1 = pl[(4 + yl) * GZ + (z + n) % GZ], c2 = pl[(4 + yl) * GZ + (z - n + GZ) % GZ];
-      v.x += c.lapt[n - 1] * (a1.x + a2.x) + c.lapt[3 + n] * (b1.x + b2.x) + c.lapt[7 + n] * (c1.x + c2.x);
-      v.y += c.lapt[n - 1] * (a1.y + a2.y) + c.lapt[3 + n] * (b1.y + b2.y) + c.lapt[7 + n] * (c1.y + c2.y);
-      w.x += nabt[n - 1] * (a1.x - a2.x) + nabt[3 + n] * (b1.x - b2.x) + nabt[7 + n] * (c1.x - c2.x);
-      w.y += nabt[n - 1] * (a1.y - a2.y) + nabt[3 + n] * (b1.y - b2.y) + nabt[7 + n] * (c1.y - c2.y);
-    }
-    // z = A e - 0.5 v - i w ;  F += conj(e) z
-    const double2 zz = make_double2(c.lap0_2 * e.x - 0.5 * v.x + w.y, c.lap0_2 * e.y - 0.5 * v.y - w.x);
-    v2[0] += e.x * zz.x + e.y * zz.y;
-    v2[1] += e.x * zz.y - e.y * zz.x;
-#pragma unroll
-    for (int m = 0; m < 8; ++m) q[m] = q[m + 1];
-    q[8] = to_d2(nxt);
-    nxt = __ldg(E + (size_t)((x + 6) % NLx) * NYZ + own);
-  }
-  block_sum<2>(v2, sh);
-  if (t == 0) {
-    out[2 * (size_t)blockIdx.x] = v2[0];
-    out[2 * (size_t)blockIdx.x + 1] = v2[1];
-  }
-}
-
 // per orbital: occ Re(tpsum) Hxyz + occ |k|^2/2 and occ sum |U|^2 iuV
 __global__ void k_energy_comb(const double* __restrict__ part, int nx, const double2* __restrict__ U,
                               const double* __restrict__ occ_o, const double* __restrict__ kAc,
@@ -957,55 +805,15 @@ __global__ void k_energy_sum(const double* __restrict__ eo, int norb, double* __
   }
 }
 
+// sgpu_energy_terms, before (one CTA per plane; 32x32 and 48x48 planes a nine-plane march) and
+// with the forward march, ms: 20^3 x 2048 orbitals complex(8) 1.24 / 0.26, 32^3 x 2048
+// complex(4) 1.08 / 0.74, 48^3 x 800 1.97 / 1.34, 16^3 x 1024 0.37 / 0.09.
 cudaError_t launch_energy(System& s, double* e_dev) {
-  double* part = s.red;                                // [norb][NLx][2]
-  double* eo = part + 2 * (size_t)s.norb * s.NLx;      // [norb][2]
-  double* coef = eo + 2 * (size_t)s.norb;              // [25]
-  if (2 * (size_t)s.norb * s.NLx + 2 * (size_t)s.norb + 32 > s.red_elems) return cudaErrorInvalidValue;
-  double h[25];
-  h[0] = -(s.lap[0][0] + s.lap[1][0] + s.lap[2][0]) * 0.5;
-  for (int d = 0; d < 3; ++d)
-    for (int n = 0; n < 4; ++n) {
-      h[1 + 4 * d + n] = s.lap[d][n + 1];
-      h[13 + 4 * d + n] = s.nab[d][n + 1];
-    }
-  cudaError_t err = cudaMemcpyAsync(coef, h, sizeof(h), cudaMemcpyHostToDevice, s.stream);
-  if (err != cudaSuccess) return err;
-  int nx = s.NLx;
-  EkinCoef ec;
-  ec.lap0_2 = h[0];
-  for (int k = 0; k < 12; ++k) {
-    ec.lapt[k] = h[1 + k];
-    ec.nab[k] = h[13 + k];
-  }
-  // 32x32 and 48x48 planes: the x-march over planes split in 8-row parts (SGPU_PARAM_CUR_FIXED)
-  if (s.cur_fixed && s.NLy == 32 && s.NLz == 32) {
-    nx = 4;
-    if (s.prec == SGPU_PREC_C64)
-      k_ekin_march_yh<float, 32, 32, 4><<<4 * s.norb, 256, 0, s.launch_stream()>>>((const float2*)s.zu, s.NLx, s.NBocc,
-                                                                                   s.kAc_d, ec, part);
-    else
-      k_ekin_march_yh<double, 32, 32, 4><<<4 * s.norb, 256, 0, s.launch_stream()>>>((const double2*)s.zu, s.NLx,
-                                                                                    s.NBocc, s.kAc_d, ec, part);
-  } else if (s.cur_fixed && s.NLy == 48 && s.NLz == 48) {
-    nx = 6;
-    if (s.prec == SGPU_PREC_C64)
-      k_ekin_march_yh<float, 48, 48, 6><<<6 * s.norb, 384, 0, s.launch_stream()>>>((const float2*)s.zu, s.NLx, s.NBocc,
-                                                                                   s.kAc_d, ec, part);
-    else
-      k_ekin_march_yh<double, 48, 48, 6><<<6 * s.norb, 384, 0, s.launch_stream()>>>((const double2*)s.zu, s.NLx,
-                                                                                    s.NBocc, s.kAc_d, ec, part);
-  } else {
-    const int gp = s.norb * s.NLx;
-    const int bt = s.NLy >= 8 ? 256 : 32 * s.NLy;
-    if (s.prec == SGPU_PREC_C64)
-      k_ekin_plane<float><<<gp, bt, 0, s.launch_stream()>>>((const float2*)s.zu, s.NLx, s.NLy, s.NLz, s.NBocc, s.kAc_d,
-                                                            coef, part);
-    else
-      k_ekin_plane<double><<<gp, bt, 0, s.launch_stream()>>>((const double2*)s.zu, s.NLx, s.NLy, s.NLz, s.NBocc,
-                                                             s.kAc_d, coef, part);
-  }
-  err = cudaGetLastError();
+  double* part = s.red;                                // [norb][nx][2], nx <= part_rows
+  double* eo = part + 2 * (size_t)s.norb * s.part_rows;  // [norb][2]
+  if (2 * (size_t)s.norb * s.part_rows + 2 * (size_t)s.norb + 32 > s.red_elems) return cudaErrorInvalidValue;
+  int nx = 1;
+  cudaError_t err = s.prec == SGPU_PREC_C64 ? fwd_march<float, true>(s, part, nx) : fwd_march<double, true>(s, part, nx);
   if (err != cudaSuccess) return err;
   // U = Hxyz * sum conj(zproj) psi = Hxyz * sum uV ekr psi  (total_energy.f90:191-197), FP64 projectors
   if (s.Nlma) {

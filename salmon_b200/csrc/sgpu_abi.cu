@@ -505,19 +505,14 @@ int sgpu_create(const sgpu_desc* d, int precision, sgpu_handle* out) {
   if ((e = dalloc(&s->vloc64, s->NL)) != cudaSuccess) return bail(cuda_fail(e, "alloc vloc64"));
   if ((e = dalloc(&s->vloc32, s->NL)) != cudaSuccess) return bail(cuda_fail(e, "alloc vloc32"));
   const size_t nchunk = (s->norb + 63) / 64;
+  s->part_rows = std::max(6, sgpu::march_blocks(s->NLy, s->NLz));  // (the fixed shapes use up to 6)
   s->red_elems = std::max<size_t>({nchunk * s->NL, 4 * (size_t)s->norb + 64, (size_t)s->NL + 64,
-                                   sgpu::current_red_elems(s->norb, s->NLx)});
+                                   sgpu::current_red_elems(s->norb, s->part_rows)});
+  if ((size_t)((s->NL + 255) / 256) * nchunk < 2 * (size_t)s->nsm)  // small grids: the density in chunks of 16 orbitals
+    s->red_elems = std::max(s->red_elems, (size_t)((s->norb + 15) / 16) * s->NL);
   if ((e = dalloc(&s->red, s->red_elems)) != cudaSuccess) return bail(cuda_fail(e, "alloc red"));
-  if ((e = dalloc(&s->cur_part, (size_t)s->norb * s->NLx * 4)) != cudaSuccess)
+  if ((e = dalloc(&s->cur_part, (size_t)s->norb * s->part_rows * 4)) != cudaSuccess)
     return bail(cuda_fail(e, "alloc cur_part"));
-  {
-    double h12[12];
-    for (int n = 0; n < 4; ++n)
-      for (int dd = 0; dd < 3; ++dd) h12[4 * dd + n] = s->nab[dd][n + 1];
-    if ((e = dalloc(&s->nab12, 12)) != cudaSuccess) return bail(cuda_fail(e, "alloc nab12"));
-    if ((e = cudaMemcpy(s->nab12, h12, sizeof(h12), cudaMemcpyHostToDevice)) != cudaSuccess)
-      return bail(cuda_fail(e, "copy nab12"));
-  }
   s->red_h_elems = (size_t)s->NL + 64;
   if ((e = cudaMallocHost((void**)&s->red_h, s->red_h_elems * sizeof(double))) != cudaSuccess)
     return bail(cuda_fail(e, "alloc pinned"));
@@ -543,7 +538,7 @@ int sgpu_destroy(sgpu_handle h) {
   free_state_buffers(s);
   void* bufs[] = {s->vloc64, s->vloc32, s->occ_o, s->kAc_d, s->idx_proj, s->atom_off, s->rpos, s->items,
                   s->lma_list, s->iuV_d, s->lma_atom, s->uV_d, s->zproj64, s->zproj32, s->sp_off, s->rec, s->cont, s->qmap, s->kbq, s->kb_multi, s->lqi, s->Sbuf, s->Wbuf,
-                  s->U, s->Up, s->Uw, s->red, s->stage, s->cur_part, s->nab12};
+                  s->U, s->Up, s->Uw, s->red, s->stage, s->cur_part};
   for (void* p : bufs) cudaFree(p);
   void* gbufs[] = {s->gs_zu, s->gs_aux, s->gs_W, s->gs_st, s->gs_part, s->gs_A, s->gs_V, s->gs_w, s->gs_sweeps,
                    s->occ_gs, s->p2_blk[0], s->p2_blk[1], s->gs_out, s->gs_R, s->gs_bad, s->gs_M, s->gs_MR, s->gs_dots, s->gs_iters, s->gs_res, s->gs_tb, s->vpsl, s->rho_d, s->exc_d, s->sp_blk,
@@ -877,7 +872,7 @@ int gs_alloc(System* s) {
   CK(cudaMalloc(&s->gs_V, (size_t)s->nkl * s->NB * s->NB * sizeof(double2)));
   CK(cudaMalloc(&s->gs_w, (size_t)s->nkl * s->NB * sizeof(double)));
   CK(cudaMalloc(&s->gs_R, (size_t)s->nkl * 32 * 32 * sizeof(double2)));
-  CK(cudaMalloc(&s->gs_bad, (size_t)s->nkl * sizeof(int)));
+  CK(cudaMalloc(&s->gs_bad, 2 * (size_t)s->nkl * sizeof(int)));
   CK(cudaMalloc(&s->gs_M, (size_t)s->nkl * s->NB * 256 * sizeof(double2)));
   CK(cudaMalloc(&s->gs_MR, (size_t)s->nkl * s->NB * 256 * sizeof(double)));
   CK(cudaMalloc(&s->gs_dots, (size_t)s->nkl * sgpu::CG_DOT_SPLITS * 256 * sizeof(double2)));

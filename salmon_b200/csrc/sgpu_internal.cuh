@@ -186,7 +186,7 @@ struct System {
   double2* gs_part = nullptr;      // [gs_part_elems] partial products of the split-K kernels
   size_t gs_part_elems = 0;
   double2* gs_R = nullptr;         // [nkl][32][32] inverse Cholesky factor of a Gram-Schmidt panel
-  int* gs_bad = nullptr;           // [nkl] panels left to the one-by-one Gram-Schmidt
+  int* gs_bad = nullptr;           // [nkl] panels left to the one-by-one Gram-Schmidt, [nkl] panels done in one round
   double2* gs_M = nullptr;         // [nkl][NB][256] rows of (I + L)^-1, L the lower bands' overlaps (k_gs.cu)
   double* gs_MR = nullptr;         // [nkl][NB][256] the same for the overlaps' real parts
   double2* gs_dots = nullptr;      // [nkl][CG_DOT_SPLITS][256] partial inner products with the lower bands
@@ -211,13 +211,13 @@ struct System {
   int* sp_blk = nullptr;           // [NLx*(nyblk+1)] first sphere point of each (plane, y-block)
   int pass_tab = 1;                // stencil pass: Vloc/sphere-index tables through the ring (two-point form)
   int pass_fixed = 1;              // stencil pass: compile-time plane shapes with a 9-plane ring (complex(4))
-  int cur_fixed = 1;               // current stencil, 32x32 / 48x48 planes: 1 two rows per thread, 2 one, 0 generic
+  int cur_fixed = 1;               // current stencil, 32x32 / 48x48 planes: 1 two rows per thread, 2 one, 0 any-shape march
   int taylor_kernel = 0;           // Taylor step: 0 auto, 1 stencil passes, 2 the shared-memory resident kernel
   // The current's stencil sums {jt, F, G, H} of the resident orbitals, computed by a
   // Taylor step called with flag_current (RT/hamiltonian.f90:68-70): rows
   // cur_part[o][cur_nx][4], valid while cur_valid (the orbitals are unchanged since).
-  double* cur_part = nullptr;      // [norb][NLx][4]
-  double* nab12 = nullptr;         // [12] nabx(1:4), naby(1:4), nabz(1:4) (device, set at creation)
+  double* cur_part = nullptr;      // [norb][part_rows][4]
+  int part_rows = 1;               // most partial rows of an orbital in the current and energy reductions
   int cur_nx = 0;
   bool cur_valid = false;
   // The stencil sums of a flag_current step run on a second stream (they only read
@@ -329,7 +329,9 @@ cudaError_t launch_psi_rho(System& s, double* rho_dev);
 cudaError_t launch_current(System& s, double* jav_dev);
 cudaError_t launch_current_proj(System& s);
 // reduction scratch (doubles) that launch_current and launch_energy need
-size_t current_red_elems(int norb, int NLx);
+size_t current_red_elems(int norb, int rows);
+// row blocks of the generic current / energy march (parts per orbital)
+int march_blocks(int NLy, int NLz);
 // per-orbital kinetic and nonlocal energies summed (device, 2 doubles)
 cudaError_t launch_energy(System& s, double* e_dev);
 

@@ -64,3 +64,18 @@ def test_density_chunks(cuda_lib, nk, nb):
     with GpuSystem(sysm) as g:
         g.set_state(zu)
         assert rel(g.psi_rho_RT(), O.psi_rho(sysm, zu)) < 1e-12
+
+
+@pytest.mark.parametrize("precision", ["c128", "c64"])
+@pytest.mark.parametrize("shape", [(9, 33, 20), (6, 5, 40), (4, 3, 7), (7, 1, 9), (3, 2, 130)])
+def test_current_and_energy_march(cuda_lib, precision, shape):
+    """Blocks of rows with an odd last one, a single row, fewer planes than the queue."""
+    from salmon_b200.rt import GpuSystem
+    sysm, kAc, vloc, zu = S.small_system(*shape, nk=2, nb=2, seed=5)
+    z = zu if precision == "c128" else zu.astype(np.complex64).astype(np.complex128)
+    with GpuSystem(sysm, precision) as g:
+        g.set_state(zu)
+        g.set_vloc(vloc)
+        jav, e = g.current_RT(kAc), g.energy_terms(kAc)
+    assert rel(jav, O.current(sysm, kAc, z)) < 1e-11  # FP64 sums in both precisions
+    assert rel(e, O.energy_terms(sysm, kAc, z)) < 1e-11
