@@ -32,6 +32,7 @@ struct GrpShared {
   double part[2][GRP_NV];    // this CTA's partial sums (double-buffered)
   double tot[GRP_NV];
   double2 dots[2][CGB];      // this CTA's inner products with the lower bands (double-buffered)
+  double2 pdots[GS_THREADS / 32][4];  // a warp's share of four of them
   double2 d[CGB], c[CGB];
 };
 
@@ -153,8 +154,8 @@ __global__ void __launch_bounds__(GS_THREADS) k_gram_schmidt(double2* __restrict
 // (I + L)^-1 grows by one row per finished band: gs_M, and gs_MR for the real parts.
 // Lower bands are taken in blocks of CGB, block after block, so one row holds the
 // CGB columns of its own block.
-// At 32^3, two k-points, 144 bands, TPA, 4 iterations: sgpu_cg + 2 Gram-Schmidt 808
-// ms with dependent sums; the measured time now stands at launch_cg_project.
+// At 32^3, two k-points, 144 bands, TPA, 4 iterations, sgpu_cg and two Gram-Schmidt: 805 ms
+// with dependent sums, now 106 ms.
 enum { CG_XK = 0, CG_HXK, CG_TXK, CG_GK, CG_PK, CG_PKO, CG_HT, CG_TT, CG_HK, CG_NW };
 
 struct CGState {
@@ -190,17 +191,28 @@ template <bool REAL>
 __device__ __forceinline__ void cg_solve(const double2* __restrict__ M, const double* __restrict__ MR, int n,
                                          const double2* d, double2* c) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int j = warp; j < n; j += nw) {
-    double2 v = make_double2(0.0, 0.0);
-    if (REAL) {
-      for (int i = lane; i <= j; i += 32) v.x = fma(MR[(size_t)j * CGB + i], d[i].x, v.x);
-      v.x = warp_sum_gs(v.x);
-    } else {
-      for (int i = lane; i <= j; i += 32) v = cfma(M[(size_t)j * CGB + i], d[i], v);
-      v.x = warp_sum_gs(v.x);
-      v.y = warp_sum_gs(v.y);
+  for (int j0 = warp; j0 < n; j0 += 4 * nw) {  // four rows of the warp at a time, their loads in flight together
+    double2 v[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) v[r] = make_double2(0.0, 0.0);
+    const int jl = min(n - 1, j0 + 3 * nw);
+    for (int i = lane; i <= jl; i += 32) {
+      const double2 di = d[i];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int j = j0 + r * nw;
+        if (j < n && i <= j) {
+          if (REAL) v[r].x = fma(MR[(size_t)j * CGB + i], di.x, v[r].x);
+          else v[r] = cfma(M[(size_t)j * CGB + i], di, v[r]);
+        }
+      }
     }
-    if (lane == 0) c[j] = v;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      v[r].x = warp_sum_gs(v[r].x);
+      if (!REAL) v[r].y = warp_sum_gs(v[r].y);
+      if (lane == 0 && j0 + r * nw < n) c[j0 + r * nw] = v[r];
+    }
   }
 }
 
@@ -219,20 +231,69 @@ __device__ __forceinline__ double2 cg_subtract(double2 x, const double2* __restr
   return x;
 }
 
-// Hxyz <u_j|x> for n bands u_j into s.d, over the cluster (ends with a CTA barrier)
+// the same at a thread's points of the CTA's slice, four points at a time (their loads are
+// in flight together)
+__device__ __forceinline__ void grp_subtract(const Grp& g, double2* x, const double2* __restrict__ u, int NL, int n,
+                                             const double2* c) {
+  int i = g.lo + threadIdx.x;
+  const int nt = blockDim.x;
+  for (; i + 3 * nt < g.hi; i += 4 * nt) {
+    double2 v[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) v[p] = x[i + p * nt];
+#pragma unroll 2
+    for (int j = 0; j < n; ++j) {
+      const double2 cj = c[j];
+      const double2* uj = u + (size_t)j * NL + i;
+#pragma unroll
+      for (int p = 0; p < 4; ++p) v[p] = csub(v[p], cmul(cj, uj[p * nt]));
+    }
+#pragma unroll
+    for (int p = 0; p < 4; ++p) x[i + p * nt] = v[p];
+  }
+  for (; i < g.hi; i += nt) x[i] = cg_subtract(x[i], u + i, NL, n, c);
+}
+
+// Hxyz <u_j|x> for n bands u_j into s.d, over the cluster (ends with a CTA barrier).  A warp
+// takes four bands (sharing the loads of x); with fewer groups of four than warps, the warps
+// of one group split the slice.
 __device__ __forceinline__ void grp_dots(Grp& g, const double2* __restrict__ u, int NL, int n, const double2* x,
                                          double Hxyz) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int ng = (n + 3) / 4, parts = max(1, nw / max(1, ng));
   double2* loc = g.s->dots[g.dparity];
   __syncthreads();  // x is written by other threads of the CTA
-  for (int j = warp; j < n; j += nw) {
-    const double2* uj = u + (size_t)j * NL;
-    double re = 0.0, im = 0.0;
+  for (int g0 = 0; g0 < ng; g0 += nw) {  // (parts > 1 only when one round takes all groups)
+    const int gi = parts > 1 ? warp % ng : g0 + warp, part = parts > 1 ? warp / ng : 0;
+    if (gi < ng && part < parts) {
+      const double2* uj = u + (size_t)4 * gi * NL;
+      const int nj = min(4, n - 4 * gi);
+      double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll 4
-    for (int i = g.lo + lane; i < g.hi; i += 32) zdot_add(re, im, uj[i], x[i]);
-    re = warp_sum_gs(re);
-    im = warp_sum_gs(im);
-    if (lane == 0) loc[j] = make_double2(re * Hxyz, im * Hxyz);
+      for (int i = g.lo + lane + 32 * part; i < g.hi; i += 32 * parts) {
+        const double2 xi = x[i];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (j < nj) zdot_add(v[2 * j], v[2 * j + 1], uj[(size_t)j * NL + i], xi);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = warp_sum_gs(v[j]) * Hxyz;
+      if (lane == 0)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (j < nj) {
+            if (parts > 1) g.s->pdots[warp][j] = make_double2(v[2 * j], v[2 * j + 1]);
+            else loc[4 * gi + j] = make_double2(v[2 * j], v[2 * j + 1]);
+          }
+    }
+  }
+  if (parts > 1) {
+    __syncthreads();
+    for (int j = threadIdx.x; j < n; j += blockDim.x) {
+      double2 t = make_double2(0.0, 0.0);
+      for (int p = 0; p < parts; ++p) t = cadd(t, g.s->pdots[p * ng + j / 4][j & 3]);
+      loc[j] = t;
+    }
   }
   if (g.C > 1) cgx::this_cluster().sync(); else __syncthreads();
   for (int j = threadIdx.x; j < n; j += blockDim.x) {
@@ -260,7 +321,7 @@ __device__ __forceinline__ void grp_project(Grp& g, const CGArgs& a, int ib, dou
     grp_dots(g, u, a.NL, n, x, a.Hxyz);
     cg_solve<REAL>(a.M + row, a.MR + row, n, g.s->d, g.s->c);
     __syncthreads();
-    GRP_FOR(i) x[i] = cg_subtract(x[i], u + i, a.NL, n, g.s->c);
+    grp_subtract(g, x, u, a.NL, n, g.s->c);
   }
 }
 
@@ -268,16 +329,35 @@ __device__ __forceinline__ void grp_project(Grp& g, const CGArgs& a, int ib, dou
 // m = -l (I + L)^-1 with l_i = <u_ib|u_i> = conj(d_i), and 1 on the diagonal.  n = ib's
 // index in its block.
 __device__ __forceinline__ void cg_new_row(double2* __restrict__ M, double* __restrict__ MR, int n, const double2* d) {
-  for (int i = threadIdx.x; i <= n; i += blockDim.x) {
-    double2 m = make_double2(i == n ? 1.0 : 0.0, 0.0);
-    double mr = m.x;
+  __shared__ double3 ps[GS_THREADS];
+  const int cols = (n + 32) / 32 * 32, parts = max(1, min(8, (int)blockDim.x / cols));  // parts of the sum per column
+  const int t = threadIdx.x;
+  for (int c0 = 0; c0 <= n; c0 += blockDim.x) {  // (one round wherever parts > 1)
+    const int i = parts > 1 ? t % cols : c0 + t, part = parts > 1 ? t / cols : 0;
+    double2 m = make_double2(0.0, 0.0);
+    double mr = 0.0;
+    if (i < n && part < parts) {
 #pragma unroll 8
-    for (int l = i; l < n; ++l) {
-      m = csub(m, cmul(make_double2(d[l].x, -d[l].y), M[(size_t)l * CGB + i]));
-      mr = fma(-d[l].x, MR[(size_t)l * CGB + i], mr);
+      for (int l = i + part; l < n; l += parts) {
+        m = csub(m, cmul(make_double2(d[l].x, -d[l].y), M[(size_t)l * CGB + i]));
+        mr = fma(-d[l].x, MR[(size_t)l * CGB + i], mr);
+      }
     }
-    M[(size_t)n * CGB + i] = m;
-    MR[(size_t)n * CGB + i] = mr;
+    if (parts > 1) {
+      ps[t] = make_double3(m.x, m.y, mr);
+      __syncthreads();
+      if (part == 0)
+        for (int p = 1; p < parts; ++p) {
+          const double3 q = ps[p * cols + i];
+          m = make_double2(m.x + q.x, m.y + q.y);
+          mr += q.z;
+        }
+    }
+    if (part == 0 && i <= n) {
+      if (i == n) { m = make_double2(1.0, 0.0); mr = 1.0; }
+      M[(size_t)n * CGB + i] = m;
+      MR[(size_t)n * CGB + i] = mr;
+    }
   }
 }
 
@@ -727,13 +807,13 @@ int cg_work_vectors() { return CG_NW; }
 // rotation R = [[c, s], [-s, c]], t = sign(tau)/(|tau|+sqrt(1+tau^2)),
 // tau = (a_qq-a_pp)/(2|b|).
 //
-// One CTA per k-point.  The 2x2 blocks (pair, pair) of A <- J^H A J and the pairs of
-// columns of V <- V J are independent, so a step is one sweep over them between two
-// barriers; A and V live in shared memory as long as both fit (JAC_SMEM), else in
-// global memory.  Bound by the chain of FP64 square roots and divisions of the next
-// step's rotations and the two barriers.
-// At 32 k-points x 40 bands: 1.05 ms with rows and columns rotated one after the
-// other in global memory; the time now stands at launch_jacobi.
+// One CTA per k-point.  The 2x2 blocks (pair, pair) of A <- J^H A J are independent: one
+// sweep over them a step, a warp per column pair.  V <- V J runs one step behind, on the
+// warps that do not compute the next step's rotations.  A and V live in shared memory as
+// long as both fit (JAC_SMEM), else in global memory.  Bound by the chain of FP64
+// reciprocal roots of a step's rotations and the two barriers.
+// At 32 k-points x 40 bands 0.53 ms; 1.05 ms with rows and columns rotated one after the
+// other in global memory, 0.64 ms with square roots and divisions in the usual order.
 //
 // Sweeps stop when the off-diagonal norm of the upper triangle, the one the rotations
 // are taken from, is below 1e-15 of the Frobenius norm, or after max_sweeps (the count
@@ -762,19 +842,19 @@ struct JacPair {
 
 constexpr size_t JAC_SMEM = 220 * 1024;
 
-static size_t jac_pair_bytes(int NB) { return (size_t)((NB + 1) / 2) * sizeof(JacPair) + (size_t)NB * (sizeof(double) + sizeof(int)); }
+static size_t jac_pair_bytes(int NB) { return 2 * (size_t)((NB + 1) / 2) * sizeof(JacPair) + (size_t)NB * (sizeof(double) + sizeof(int)); }
 
 __global__ void __launch_bounds__(1024) k_jacobi_herm(double2* __restrict__ Aall, double2* __restrict__ Vall, int NB,
                                                       int max_sweeps, int in_smem, double* __restrict__ w,
                                                       int* __restrict__ sweeps) {
   extern __shared__ __align__(16) unsigned char jraw[];
   const int n = NB + (NB & 1), nh = n / 2;  // even count for the round-robin (index NB is a dummy)
-  JacPair* pr = reinterpret_cast<JacPair*>(jraw);           // [nh]
-  double* ev = reinterpret_cast<double*>(pr + nh);          // [NB] eigenvalues
+  JacPair* pr2 = reinterpret_cast<JacPair*>(jraw);          // [2][nh], this step's and the previous one's
+  double* ev = reinterpret_cast<double*>(pr2 + 2 * nh);     // [NB] eigenvalues
   int* rank = reinterpret_cast<int*>(ev + NB);              // [NB]
   double2* mats = reinterpret_cast<double2*>(jraw + (((size_t)((unsigned char*)(rank + NB) - jraw) + 15) & ~(size_t)15));
   __shared__ double sh[64];
-  const int k = blockIdx.x, t = threadIdx.x, nt = blockDim.x;
+  const int k = blockIdx.x, t = threadIdx.x, nt = blockDim.x, lane = t & 31, warp = t >> 5, nwarp = nt >> 5;
   double2* Ag = Aall + (size_t)k * NB * NB;
   double2* Vg = Vall + (size_t)k * NB * NB;
   double2* A = in_smem ? mats : Ag;
@@ -798,36 +878,59 @@ __global__ void __launch_bounds__(1024) k_jacobi_herm(double2* __restrict__ Aall
     const double fro2 = v[0] + 2.0 * v[1];
     if (2.0 * v[1] <= 1e-30 * fro2) break;
     const double tiny2 = 1e-50 * fro2;
-    for (int step = 0; step < n - 1; ++step) {
-      for (int i = t; i < nh; i += nt) {
-        // ring position i pairs with n-1-i (i = 0: the fixed index)
-        const int q0 = i == 0 ? 0 : 1 + (i + step) % (n - 1), q1 = rr_partner(q0, step, n);
-        JacPair j;
-        j.p = min(q0, q1);
-        j.q = max(q0, q1) < NB ? max(q0, q1) : -1;
-        j.c = 1.0;
-        j.s = 0.0;
-        j.eph = make_double2(1.0, 0.0);
-        if (j.q >= 0) {
-          const double app = AE(j.p, j.p).x, aqq = AE(j.q, j.q).x;
-          const double2 b = AE(j.p, j.q);
-          const double m2 = b.x * b.x + b.y * b.y;
-          if (m2 > tiny2 && m2 > 1e-290) {
-            const double ab = sqrt(m2);
-            const double tau = (aqq - app) / (2.0 * ab);
-            const double tt = (tau >= 0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-            j.c = 1.0 / sqrt(1.0 + tt * tt);
-            j.s = tt * j.c;
-            j.eph = make_double2(b.x / ab, b.y / ab);
+    for (int step = 0; step <= n - 1; ++step) {
+      JacPair* pr = pr2 + (step & 1) * nh;
+      const JacPair* prev = pr2 + ((step & 1) ^ 1) * nh;
+      const int npw = (nh + 31) / 32;  // warps that compute rotations
+      if (warp < npw && step < n - 1) {
+        for (int i = t; i < nh; i += 32 * npw) {
+          // ring position i pairs with n-1-i (i = 0: the fixed index)
+          const int q0 = i == 0 ? 0 : 1 + (i + step) % (n - 1), q1 = rr_partner(q0, step, n);
+          JacPair j;
+          j.p = min(q0, q1);
+          j.q = max(q0, q1) < NB ? max(q0, q1) : -1;
+          j.c = 1.0;
+          j.s = 0.0;
+          j.eph = make_double2(1.0, 0.0);
+          if (j.q >= 0) {
+            const double app = AE(j.p, j.p).x, aqq = AE(j.q, j.q).x;
+            const double2 b = AE(j.p, j.q);
+            const double m2 = b.x * b.x + b.y * b.y;
+            if (m2 > tiny2 && m2 > 1e-290) {
+              // with delta = (a_qq - a_pp) / 2 and h = sqrt(delta^2 + |b|^2): c^2 = (1 + |delta| / h) / 2,
+              // s = sign(delta) |b| / (2 c h), the same rotation from two reciprocal roots in a row
+              const double del = 0.5 * (aqq - app);
+              const double ih = rsqrt(fma(del, del, m2)), iab = rsqrt(m2);
+              const double c2 = fma(0.5 * fabs(del), ih, 0.5), ic = rsqrt(c2);
+              j.c = c2 * ic;
+              j.s = (del >= 0 ? 0.5 : -0.5) * (m2 * iab) * ih * ic;
+              j.eph = make_double2(b.x * iab, b.y * iab);
+            }
+          }
+          pr[i] = j;
+        }
+      }
+      if (step > 0 && (warp >= npw || step == n - 1 || npw >= nwarp)) {  // V <- V J of the previous step
+        const int w0 = step == n - 1 || npw >= nwarp ? 0 : npw;
+        for (int f = warp - w0; f < nh; f += nwarp - w0) {
+          const JacPair b = prev[f];
+          if (b.q < 0) continue;
+          const double2 em = make_double2(b.eph.x, -b.eph.y);
+          for (int row = lane; row < NB; row += 32) {
+            const double2 xp = VE(row, b.p), ex = cmul(em, VE(row, b.q));
+            VE(row, b.p) = make_double2(b.c * xp.x - b.s * ex.x, b.c * xp.y - b.s * ex.y);
+            VE(row, b.q) = make_double2(b.s * xp.x + b.c * ex.x, b.s * xp.y + b.c * ex.y);
           }
         }
-        pr[i] = j;
       }
       __syncthreads();
-      // A <- J^H A J, block by block; V <- V J, row by row
-      for (int e = t; e < nh * nh + nh * NB; e += nt) {
-        if (e < nh * nh) {
-          const JacPair a = pr[e % nh], b = pr[e / nh];
+      if (step == n - 1) break;
+      // A <- J^H A J, block by block: a warp per column pair, lanes over row pairs
+      for (int jb = warp; jb < nh; jb += nwarp) {
+        const JacPair b = pr[jb];
+        const double2 em = make_double2(b.eph.x, -b.eph.y);
+        for (int ja = lane; ja < nh; ja += 32) {
+          const JacPair a = pr[ja];
           const int rows[2] = {a.p, a.q}, cols[2] = {b.p, b.q};
           double2 x[2][2];
 #pragma unroll
@@ -841,7 +944,6 @@ __global__ void __launch_bounds__(1024) k_jacobi_herm(double2* __restrict__ Aall
             x[0][j] = make_double2(a.c * xp.x - a.s * ex.x, a.c * xp.y - a.s * ex.y);
             x[1][j] = make_double2(a.s * xp.x + a.c * ex.x, a.s * xp.y + a.c * ex.y);
           }
-          const double2 em = make_double2(b.eph.x, -b.eph.y);
 #pragma unroll
           for (int i = 0; i < 2; ++i) {  // columns: new_p = c x_p - s e^{-i phi} x_q, new_q = s x_p + c e^{-i phi} x_q
             const double2 ex = cmul(em, x[i][1]), xp = x[i][0];
@@ -853,14 +955,6 @@ __global__ void __launch_bounds__(1024) k_jacobi_herm(double2* __restrict__ Aall
 #pragma unroll
             for (int j = 0; j < 2; ++j)
               if (rows[i] >= 0 && cols[j] >= 0) AE(rows[i], cols[j]) = x[i][j];
-        } else {
-          const int f = e - nh * nh, row = f % NB;
-          const JacPair b = pr[f / NB];
-          if (b.q >= 0) {
-            const double2 xp = VE(row, b.p), ex = cmul(make_double2(b.eph.x, -b.eph.y), VE(row, b.q));
-            VE(row, b.p) = make_double2(b.c * xp.x - b.s * ex.x, b.c * xp.y - b.s * ex.y);
-            VE(row, b.q) = make_double2(b.s * xp.x + b.c * ex.x, b.s * xp.y + b.c * ex.y);
-          }
         }
       }
       __syncthreads();
@@ -895,7 +989,8 @@ cudaError_t launch_jacobi(const System& s, double2* A, double2* V, int max_sweep
     const cudaError_t e = raise_smem_limit((const void*)k_jacobi_herm, smem);
     if (e != cudaSuccess) return e;
   }
-  k_jacobi_herm<<<s.nkl, 1024, smem, s.launch_stream()>>>(A, V, s.NB, max_sweeps, in_smem, w, sweeps);
+  const int nt = 32 * std::min(32, std::max(8, (s.NB + 1) / 2 + 1));  // a warp per column pair, and one for the rotations
+  k_jacobi_herm<<<s.nkl, nt, smem, s.launch_stream()>>>(A, V, s.NB, max_sweeps, in_smem, w, sweeps);
   return cudaGetLastError();
 }
 

@@ -26,16 +26,17 @@ __device__ __forceinline__ void zmma(double (&d)[2], double a, double b) {
 // chunks of 8 points through a four-stage cp.async ring (rows padded to 10 values:
 // the eight rows a warp reads fall in distinct banks, two wavefronts a load).
 // lower: tiles above the diagonal are skipped (Hermitian products).
-// Bound by the FP64 pipe: 8 MMAs per 4 shared-memory loads.  At 16x16x32, 32 k,
-// 40 bands (the CUDA-core form with 16 x 16 tiles in brackets): see launch_subspace_h.
+// Bound by the FP64 pipe: 8 MMAs per 4 shared-memory loads.  At 16x16x32, 32 k, 40 bands:
+// H_sub 0.25 ms (CUDA cores, 16 x 16 tiles: 0.51), the rotation 0.14 ms (0.45).
 constexpr int ZT = 32, ZK = 8, ZROW = ZK + 2, ZST = 4;
 
 __global__ void __launch_bounds__(128) k_zgemm_hn(const double2* __restrict__ A, const double2* __restrict__ B,
                                                  size_t kstride, int M, int N, int NL, int kchunk, int tm_count,
-                                                 int lower, double2* __restrict__ part) {
+                                                 int lower, const int* __restrict__ skip, double2* __restrict__ part) {
   __shared__ double2 sa[ZST][ZT][ZROW], sb[ZST][ZT][ZROW];
   const int k = blockIdx.x / tm_count, tm = blockIdx.x - k * tm_count, tn = blockIdx.y;
   if (lower && tm < tn) return;  // whole CTA
+  if (skip && skip[k]) return;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int i0 = blockIdx.z * kchunk, i1 = min(i0 + kchunk, NL);
   const double2* Ak = A + k * kstride + (size_t)tm * ZT * NL;
@@ -59,6 +60,14 @@ __global__ void __launch_bounds__(128) k_zgemm_hn(const double2* __restrict__ A,
   };
   const int wm = (warp & 1) * 16, wn = (warp >> 1) * 16;
   const int row = lane >> 2, pt = (lane >> 1) & 1, prt = lane & 1;
+  // the warp's 8 x 8 sub-tiles with an element to compute (uniform over the warp)
+  bool need[2][2];
+#pragma unroll
+  for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+    for (int ni = 0; ni < 2; ++ni)
+      need[mi][ni] = wm + 8 * mi < mrows && wn + 8 * ni < nrows && !(lower && tm == tn && wm + 8 * mi + 7 < wn + 8 * ni);
+  const bool any = need[0][0] || need[0][1] || need[1][0] || need[1][1];
   double cre[2][2][2] = {}, cim[2][2][2] = {};
   for (int c = 0; c < ZST - 1; ++c) issue(c);
   for (int c = 0; c < nch; ++c) {
@@ -66,6 +75,7 @@ __global__ void __launch_bounds__(128) k_zgemm_hn(const double2* __restrict__ A,
     __syncthreads();
     issue(c + ZST - 1);
     const int s = c % ZST;
+    if (!any) continue;
 #pragma unroll
     for (int ks = 0; ks < ZK / 2; ++ks) {
       const int p = 2 * ks + pt;
@@ -81,8 +91,10 @@ __global__ void __launch_bounds__(128) k_zgemm_hn(const double2* __restrict__ A,
       for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
         for (int ni = 0; ni < 2; ++ni) {
-          zmma(cre[mi][ni], a[mi], br[ni]);
-          zmma(cim[mi][ni], a[mi], bi[ni]);
+          if (need[mi][ni]) {
+            zmma(cre[mi][ni], a[mi], br[ni]);
+            zmma(cim[mi][ni], a[mi], bi[ni]);
+          }
         }
     }
   }
@@ -111,9 +123,10 @@ constexpr int ZP = 64, ZST2 = 3;
 
 __global__ void __launch_bounds__(128) k_zgemm_nn(const double2* X, size_t xstride, const double2* __restrict__ Z,
                                                  size_t zstride, int ldz, int M, int N, int NL, const double2* base,
-                                                 double2* out, size_t ostride) {
+                                                 double2* out, size_t ostride, const int* __restrict__ skip) {
   __shared__ double2 sx[ZST2][ZK][ZP], sz[ZST2][ZT][ZROW];
   const int k = blockIdx.z, n0 = blockIdx.y * ZT, p0 = blockIdx.x * ZP;
+  if (skip && skip[k]) return;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const double2* Xk = X + k * xstride;
   const double2* Zk = Z + k * zstride;
@@ -152,6 +165,7 @@ __global__ void __launch_bounds__(128) k_zgemm_nn(const double2* X, size_t xstri
       for (int h = 0; h < 2; ++h) a[h] = reinterpret_cast<const double*>(&sx[s][r][16 * warp + 8 * h + row])[prt];
 #pragma unroll
       for (int ni = 0; ni < 4; ++ni) {
+        if (n0 + 8 * ni >= N) continue;  // uniform
         const double2 z = sz[s][8 * ni + row][r];
         const double br = prt ? -z.y : z.x, bi = prt ? z.x : z.y;
 #pragma unroll
@@ -192,20 +206,20 @@ static int zsplit(const System& s, int tiles, size_t mn) {
 }
 
 static cudaError_t launch_hn(const System& s, const double2* A, int M, const double2* B, int N, bool lower,
-                             double2* part, int& nsplit) {
+                             double2* part, int& nsplit, const int* skip = nullptr) {
   const int tm = (M + ZT - 1) / ZT, tn = (N + ZT - 1) / ZT;
   nsplit = zsplit(s, lower ? tm * (tm + 1) / 2 : tm * tn, (size_t)M * N);
   const int kchunk = ((s.NL + nsplit - 1) / nsplit + ZK - 1) / ZK * ZK;
   k_zgemm_hn<<<dim3(s.nkl * tm, tn, nsplit), 128, 0, s.launch_stream()>>>(A, B, (size_t)s.NB * s.NL, M, N, s.NL,
-                                                                         kchunk, tm, lower ? 1 : 0, part);
+                                                                         kchunk, tm, lower ? 1 : 0, skip, part);
   return cudaGetLastError();
 }
 
 static cudaError_t launch_nn(const System& s, const double2* X, int M, const double2* Z, size_t zstride, int ldz, int N,
-                             const double2* base, double2* out) {
+                             const double2* base, double2* out, const int* skip = nullptr) {
   const size_t ks = (size_t)s.NB * s.NL;
   k_zgemm_nn<<<dim3((s.NL + ZP - 1) / ZP, (N + ZT - 1) / ZT, s.nkl), 128, 0, s.launch_stream()>>>(
-      X, ks, Z, zstride, ldz, M, N, s.NL, base, out, ks);
+      X, ks, Z, zstride, ldz, M, N, s.NL, base, out, ks, skip);
   return cudaGetLastError();
 }
 
@@ -253,27 +267,31 @@ cudaError_t launch_rotate(const System& s, const double2* in, const double2* Z, 
 // The reference projects each band on the lower ones one by one
 // (GS/Gram_Schmidt.f90:32-55), i.e. builds the QR factorisation with a positive
 // diagonal by modified Gram-Schmidt: NB (NB-1) / 2 dependent inner products.
-// Here panels of 32 bands are orthonormalised through their Gram matrix, then
+// Here panels of up to 32 bands are orthonormalised through their Gram matrix, then
 // projected out of all later bands at once (modified Gram-Schmidt by blocks):
 //   S = P^H P, S = L L^H, P <- P L^-H, twice (CholeskyQR2: Yamamoto, Nakatsukasa,
 //   Yanagisawa and Fukaya, ETNA 44 (2015) 306: orthogonal to working precision for
 //   condition numbers up to ~1e8), then X <- X - P (P^H X) for the later bands.
+// A panel whose pivots all stay above GS_ONCE of their diagonal entries needs no second
+// round: the first leaves it orthonormal to eps times its squared condition number, here a few.
 // The factorisation is unique, so the result is the reference's up to rounding.  A
 // panel whose Cholesky meets a pivot below 1e-9 of its diagonal entry (bands
 // dependent to 3e-5), a zero or a NaN is left to k_gram_schmidt, the one-by-one
-// form, for that k-point.
+// form, for that k-point.  One Gram-Schmidt at 16x16x32, 32 k, 40 bands: 3.56 -> 0.5 ms.
 constexpr int GSP = 32;  // bands of a panel, = the output tile of k_zgemm_nn (in place)
-constexpr double GS_PIVOT = 1e-9;
+constexpr double GS_PIVOT = 1e-9, GS_ONCE = 0.25;
 
 // Sums the panel's Gram matrix, factors it and writes Z[k][n][m] = (L^-H)(m, n):
 // one CTA per k-point, thread (i, l) owns element (i, l) of the trailing matrix and
 // of L^-1 (eliminated together, one barrier a column).
 __global__ void __launch_bounds__(GSP* GSP) k_gs_chol(const double2* __restrict__ part, int nsplit, int nkl, int pb,
                                                       double Hxyz, int round, int* __restrict__ bad,
-                                                      double2* __restrict__ Z) {
+                                                      int* __restrict__ once, double2* __restrict__ Z) {
   __shared__ double2 A[GSP][GSP + 1], W[GSP][GSP + 1];
   __shared__ double d0[GSP], inv[GSP];
   const int k = blockIdx.x, i = threadIdx.x / GSP, l = threadIdx.x % GSP;
+  if (round == 1 && once[k]) return;  // (the products of this round return too)
+  bool good = true;
   double2 a = make_double2(0.0, 0.0);
   if (i < pb && l <= i)
     for (int sp = 0; sp < nsplit; ++sp) {
@@ -291,6 +309,7 @@ __global__ void __launch_bounds__(GSP* GSP) k_gs_chol(const double2* __restrict_
     const double d = A[j][j].x;
     ok = d > GS_PIVOT * d0[j] && d > 0.0 && d < 1e300;  // the same for every thread; false for NaN
     if (!ok) break;
+    good = good && d > GS_ONCE * d0[j];
     const double r = 1.0 / sqrt(d);
     if (threadIdx.x == 0) inv[j] = r;
     if (i > j && i < pb) {
@@ -310,8 +329,12 @@ __global__ void __launch_bounds__(GSP* GSP) k_gs_chol(const double2* __restrict_
     Z[((size_t)k * GSP + i) * GSP + l] = z;
   }
   if (threadIdx.x == 0) {
-    if (round == 0) bad[k] = ok ? 0 : 1;
-    else if (!ok) bad[k] = 1;
+    if (round == 0) {
+      bad[k] = ok ? 0 : 1;
+      once[k] = ok && good ? 1 : 0;
+    } else if (!ok) {
+      bad[k] = 1;
+    }
   }
 }
 
@@ -331,15 +354,19 @@ __global__ void k_part_sum(const double2* __restrict__ part, int nsplit, size_t 
 
 cudaError_t launch_gram_schmidt(const System& s, double2* zu) {
   cudaError_t e;
-  for (int p0 = 0; p0 < s.NB; p0 += GSP) {
-    const int pb = std::min(GSP, s.NB - p0), rest = s.NB - p0 - pb;
+  const int npan = (s.NB + GSP - 1) / GSP, pw = (s.NB + npan - 1) / npan;  // panels of equal width
+  for (int p0 = 0; p0 < s.NB; p0 += pw) {
+    const int pb = std::min(pw, s.NB - p0), rest = s.NB - p0 - pb;
     double2* P = zu + (size_t)p0 * s.NL;
     int ns = 1;
+    int* once = s.gs_bad + s.nkl;
     for (int round = 0; round < 2; ++round) {
-      if ((e = launch_hn(s, P, pb, P, pb, true, s.gs_part, ns)) != cudaSuccess) return e;
-      k_gs_chol<<<s.nkl, GSP * GSP, 0, s.launch_stream()>>>(s.gs_part, ns, s.nkl, pb, s.Hxyz, round, s.gs_bad, s.gs_R);
+      const int* skip = round ? once : nullptr;
+      if ((e = launch_hn(s, P, pb, P, pb, true, s.gs_part, ns, skip)) != cudaSuccess) return e;
+      k_gs_chol<<<s.nkl, GSP * GSP, 0, s.launch_stream()>>>(s.gs_part, ns, s.nkl, pb, s.Hxyz, round, s.gs_bad, once,
+                                                            s.gs_R);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
-      if ((e = launch_nn(s, P, pb, s.gs_R, (size_t)GSP * GSP, GSP, pb, nullptr, P)) != cudaSuccess) return e;
+      if ((e = launch_nn(s, P, pb, s.gs_R, (size_t)GSP * GSP, GSP, pb, nullptr, P, skip)) != cudaSuccess) return e;
     }
     if ((e = launch_gram_schmidt_panel(s, zu, p0, pb, s.gs_bad)) != cudaSuccess) return e;
     if (rest > 0) {
