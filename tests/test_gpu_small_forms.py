@@ -79,3 +79,42 @@ def test_current_and_energy_march(cuda_lib, precision, shape):
         jav, e = g.current_RT(kAc), g.energy_terms(kAc)
     assert rel(jav, O.current(sysm, kAc, z)) < 1e-11  # FP64 sums in both precisions
     assert rel(e, O.energy_terms(sysm, kAc, z)) < 1e-11
+
+
+@pytest.mark.parametrize("precision", ["c128", "c64"])
+@pytest.mark.parametrize("shape,nslab", [((3, 32, 32), 1), ((10, 32, 32), 3), ((7, 48, 48), 2), ((5, 16, 32), 1),
+                                         ((4, 16, 16), 1)])
+def test_two_row_pass(cuda_lib, precision, shape, nslab):
+    """Planes with a two-row form: fewer planes than the queue, x-slabs, the H application too."""
+    from salmon_b200.rt import GpuSystem
+    sysm, kAc, vloc, zu = S.small_system(*shape, nk=1, nb=3, a=(shape[0] * 0.5, 9.0, 9.5), seed=3)
+    _, zproj = O.update_projector(sysm, kAc)
+    z_in = zu if precision == "c128" else zu.astype(np.complex64).astype(np.complex128)
+    with GpuSystem(sysm, precision) as g:
+        g.set_param("taylor_kernel", 1)
+        g.set_param("nslab", nslab)
+        g.set_state(zu)
+        g.set_vloc(vloc)
+        g.update_projector(kAc)
+        g.hamiltonian(0.004)
+        assert rel(g.get_state(), O.hamiltonian(sysm, kAc, vloc, zproj, 0.004, z_in)) < TOL[precision]
+        h, tt = g.hpsi_omp_KB_GS(1, z_in[0, 2])
+    h_ref, tt_ref = O.hpsi(sysm, kAc, vloc, zproj, 1, z_in[0, 2], want_tt=True)
+    assert rel(h, h_ref) < TOL[precision] and rel(tt, tt_ref) < TOL[precision]
+
+
+@pytest.mark.parametrize("precision", ["c128", "c64"])
+@pytest.mark.parametrize("nb,rps", [(1, 0.7), (5, 1.6), (35, 1.6), (33, 2.4)])
+def test_whole_atom_projections(cuda_lib, precision, nb, rps):
+    """Atoms staged whole: ragged band groups, points in two spheres, atoms of few points."""
+    from salmon_b200.rt import GpuSystem
+    sysm, kAc, vloc, zu = S.small_system(8, 10, 12, nk=2, nb=nb, Rps=rps, seed=9)
+    _, zproj = O.update_projector(sysm, kAc)
+    z_in = zu if precision == "c128" else zu.astype(np.complex64).astype(np.complex128)
+    with GpuSystem(sysm, precision) as g:
+        g.set_param("taylor_kernel", 1)
+        g.set_state(zu)
+        g.set_vloc(vloc)
+        g.update_projector(kAc)
+        g.hamiltonian(0.02)
+        assert rel(g.get_state(), O.hamiltonian(sysm, kAc, vloc, zproj, 0.02, z_in)) < TOL[precision]
