@@ -36,9 +36,9 @@ sys.path.insert(0, ROOT)
 METRIC = "RT orbital-updates/s: FP32+FP64-reduce vs FP64 GPU at ΔJ<1e-5; hpsi %HBM peak"
 DT = 0.08
 # ncu dram__bytes_read.sum + dram__bytes_write.sum of one Taylor-stage launch, per
-# orbital, from the capture in profiles/k_hpsi_pass_stage_c64_32cubed_864orb.md
-# (864 orbitals; traffic grows with the orbital count).
-NCU_TRAFFIC_BYTES_PER_ORBITAL = {("taylor_stage", "c64", 32): 534.936064e6 / 864}
+# orbital, from the capture in profiles/k_hpsi_pass2_c64_c128.md (512 orbitals;
+# traffic grows with the orbital count).
+NCU_TRAFFIC_BYTES_PER_ORBITAL = {("taylor_stage", "c64", 32): 337.961472e6 / 512}
 
 
 def parse():
@@ -720,7 +720,7 @@ def main():
             "step_gbs_algorithmic": {p: res[p]["step_gbs"] for p in res},
             "roofline": {"bound": "hbm", "achieved": h["achieved_gbs"], "peak": hbm_peak, "unit": "GB/s",
                          "frac": h["achieved_gbs"] / hbm_peak, "traffic": traffic,
-                         "kernel": "k_hpsi_pass<float,2,2> (one Taylor stage psi + c H psi, all orbitals)",
+                         "kernel": "k_hpsi_pass2<float,2> (one Taylor stage psi + c H psi, all orbitals)",
                          "peak_kind": peak_kind},
             "cpu_baseline": cpu,
             "e2e": h["e2e"],
