@@ -384,9 +384,10 @@ int sgpu_autotune(sgpu_handle h, int reps, int* nslab, int* split, double* ms_pe
  * (SGPU_PARAM_TAYLOR_KERNEL 2 where the resident form fits, else 1), and for
  * the stencil passes the compile-time plane shapes (SGPU_PARAM_PASS_FIXED),
  * the table staging (SGPU_PARAM_PASS_TABLES), x-slabs (SGPU_PARAM_NSLAB 1, 2,
- * 4) and the KB kernel (tile, split tile with its automatic point ranges, or
- * band quad with split 1, 2, 4, 8).  Keeps the
- * fastest in the handle.  params (HOST [6], may be NULL) receives
+ * 4) and the KB kernel (the library's choice, tile, split tile with its
+ * automatic point ranges, or band quad with split 1, 2, 4, 8); and the form the
+ * handle takes with every parameter at its default.  Keeps the fastest in the
+ * handle.  params (HOST [6], may be NULL) receives
  * {taylor_kernel, pass_fixed, pass_tables, nslab, kb_kernel, uvpsi_split};
  * ms_per_step (may be NULL) its time.  The resident orbitals are not modified.
  * No reference counterpart; the nearest is auto_blocking

@@ -210,7 +210,7 @@ struct System {
   int* p2_blk[2] = {nullptr, nullptr};
   int* sp_blk = nullptr;           // [NLx*(nyblk+1)] first sphere point of each (plane, y-block)
   int pass_tab = 1;                // stencil pass: Vloc/sphere-index tables through the ring (two-point form)
-  int pass_fixed = 1;              // stencil pass: compile-time plane shapes with a 9-plane ring (complex(4))
+  int pass_fixed = 1;              // stencil pass: compile-time plane shapes (two rows per thread, or constant ring offsets)
   int cur_fixed = 1;               // current stencil, 32x32 / 48x48 planes: 1 two rows per thread, 2 one, 0 any-shape march
   int taylor_kernel = 0;           // Taylor step: 0 auto, 1 stencil passes, 2 the shared-memory resident kernel
   // The current's stencil sums {jt, F, G, H} of the resident orbitals, computed by a
