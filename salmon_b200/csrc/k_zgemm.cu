@@ -272,14 +272,23 @@ cudaError_t launch_rotate(const System& s, const double2* in, const double2* Z, 
 //   S = P^H P, S = L L^H, P <- P L^-H, twice (CholeskyQR2: Yamamoto, Nakatsukasa,
 //   Yanagisawa and Fukaya, ETNA 44 (2015) 306: orthogonal to working precision for
 //   condition numbers up to ~1e8), then X <- X - P (P^H X) for the later bands.
-// A panel whose pivots all stay above GS_ONCE of their diagonal entries needs no second
-// round: the first leaves it orthonormal to eps times its squared condition number, here a few.
-// The factorisation is unique, so the result is the reference's up to rounding.  A
-// panel whose Cholesky meets a pivot below 1e-9 of its diagonal entry (bands
-// dependent to 3e-5), a zero or a NaN is left to k_gram_schmidt, the one-by-one
-// form, for that k-point.  One Gram-Schmidt at 16x16x32, 32 k, 40 bands: 3.56 -> 0.5 ms.
+// Which rounds a panel gets follows from tau = sum |(D^1/2 L^-H)_ml|^2, D the diagonal of S:
+// tau bounds the largest eigenvalue of the inverse of the panel's scaled Gram matrix, whose
+// trace is pb, so the squared condition number of the scaled bands is at most pb tau.  (The
+// pivots bound nothing of the kind: bands that each overlap with the one before keep pivots of
+// a quarter while the condition number grows like 1.7^pb.)
+//   tau <= GS_ONCE pb (orthogonal bands have tau = pb): one round leaves the panel
+//     orthonormal to a few eps; the bands of a running ground state are here.
+//   tau <= GS_COND: two rounds, the first leaving an error of at most about 1e-16 pb tau <
+//     1e-3, which the second squares away; it has to find tau <= GS_ONCE pb itself.
+//   beyond, or a pivot below GS_PIVOT of its diagonal entry, a zero or a NaN: k_gram_schmidt,
+//     the one-by-one form, for that k-point.
+// The factorisation is unique, so the result is the reference's up to rounding.  Largest
+// |<u_i|u_j> - delta_ij|, 32 bands with a sine of 0.51 / 0.6 / 0.8 to the band before: one by
+// one 1e-8 / 3e-12 / 2e-15, here 1e-8 (one by one) / 6e-16 (two rounds) / 9e-16.
+// One Gram-Schmidt at 16x16x32, 32 k, 40 bands: 3.56 -> 0.5 ms.
 constexpr int GSP = 32;  // bands of a panel, = the output tile of k_zgemm_nn (in place)
-constexpr double GS_PIVOT = 1e-9, GS_ONCE = 0.25;
+constexpr double GS_PIVOT = 1e-9, GS_ONCE = 2.0, GS_COND = 1e11;
 
 // Sums the panel's Gram matrix, factors it and writes Z[k][n][m] = (L^-H)(m, n):
 // one CTA per k-point, thread (i, l) owns element (i, l) of the trailing matrix and
@@ -288,10 +297,9 @@ __global__ void __launch_bounds__(GSP* GSP) k_gs_chol(const double2* __restrict_
                                                       double Hxyz, int round, int* __restrict__ bad,
                                                       int* __restrict__ once, double2* __restrict__ Z) {
   __shared__ double2 A[GSP][GSP + 1], W[GSP][GSP + 1];
-  __shared__ double d0[GSP], inv[GSP];
+  __shared__ double d0[GSP], inv[GSP], sh[32];
   const int k = blockIdx.x, i = threadIdx.x / GSP, l = threadIdx.x % GSP;
   if (round == 1 && once[k]) return;  // (the products of this round return too)
-  bool good = true;
   double2 a = make_double2(0.0, 0.0);
   if (i < pb && l <= i)
     for (int sp = 0; sp < nsplit; ++sp) {
@@ -309,7 +317,6 @@ __global__ void __launch_bounds__(GSP* GSP) k_gs_chol(const double2* __restrict_
     const double d = A[j][j].x;
     ok = d > GS_PIVOT * d0[j] && d > 0.0 && d < 1e300;  // the same for every thread; false for NaN
     if (!ok) break;
-    good = good && d > GS_ONCE * d0[j];
     const double r = 1.0 / sqrt(d);
     if (threadIdx.x == 0) inv[j] = r;
     if (i > j && i < pb) {
@@ -323,6 +330,11 @@ __global__ void __launch_bounds__(GSP* GSP) k_gs_chol(const double2* __restrict_
     }
   }
   __syncthreads();
+  double tau[1] = {0.0};
+  if (ok && i < pb && l <= i) tau[0] = (W[i][l].x * W[i][l].x + W[i][l].y * W[i][l].y) * inv[i] * inv[i] * d0[l];
+  block_allsum<1>(tau, sh);
+  const bool good = tau[0] <= GS_ONCE * pb;  // the same in every thread; false for NaN
+  ok = ok && (good || (round == 0 && tau[0] <= GS_COND));
   if (i < pb && l < pb) {
     double2 z = make_double2(i == l ? 1.0 : 0.0, 0.0);  // a refused panel: left as it is
     if (ok) z = l <= i ? make_double2(W[i][l].x * inv[i], -W[i][l].y * inv[i]) : make_double2(0.0, 0.0);

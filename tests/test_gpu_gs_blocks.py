@@ -63,6 +63,42 @@ def test_gram_schmidt_dependent_and_zero_bands(cuda_lib):
     assert rel(out[2, :4], ref[2, :4]) < 1e-12
 
 
+def orthonormality(sysm, out):
+    ov = np.einsum("kbi,kci->kbc", out.conj(), out) * sysm.Hxyz
+    return np.abs(ov - np.eye(out.shape[1])).max()
+
+
+@pytest.mark.parametrize("nb,sine", [(32, 0.51), (32, 0.55), (24, 0.51), (32, 0.6), (33, 0.6), (32, 0.8), (32, 0.99)])
+def test_gram_schmidt_correlated_bands(cuda_lib, nb, sine):
+    """Bands that each overlap with the one before: the distance to the earlier bands stays
+    `sine` while the condition number grows like ((1 + cosine) / sine)^nb at worst.  Not worse
+    than the one-by-one form, whose loss of orthogonality is a few eps * kappa."""
+    sysm, kAc, vloc, z = raw_system((7, 9, 11), 2, nb)
+    for k in range(2):
+        q = np.linalg.qr(z[k].T)[0].T
+        z[k, 0] = q[0]
+        z[k, 1:] = np.sqrt(1 - sine**2) * q[:-1] + sine * q[1:]
+    kappa = max(np.linalg.cond(z[k]) for k in range(2))
+    out = gram_schmidt(sysm, kAc, vloc, z)
+    eps = np.finfo(float).eps
+    assert orthonormality(sysm, out) < 4 * eps * kappa + 1e-14
+    assert rel(out, O.gram_schmidt(sysm, z)) < 20 * eps * kappa + 1e-13
+
+
+@pytest.mark.parametrize("eps", [1e-1, 1e-2, 1e-3, 1e-4])
+def test_gram_schmidt_second_round(cuda_lib, eps):
+    """One close pair: a condition number of about 1 / eps, which the second round takes out
+    within a panel; what is left of the first panel in the second one's bands is rounding
+    over eps, as one by one."""
+    sysm, kAc, vloc, z = raw_system((7, 9, 11), 2, 40)
+    z[0, 5] = z[0, 3] + eps * z[0, 5]
+    z[1, 36] = z[1, 34] + eps * z[1, 36]
+    out = gram_schmidt(sysm, kAc, vloc, z)
+    assert orthonormality(sysm, out[:1]) < 1e-14
+    assert orthonormality(sysm, out) < 1e-15 / eps + 1e-14
+    assert rel(out, O.gram_schmidt(sysm, z)) < 1e-14 / eps + 1e-13
+
+
 @pytest.mark.parametrize("grid,nk,nb,orthonormal", [
     ((7, 9, 11), 2, 9, False),      # bands not orthogonal: the order of the projections counts
     ((8, 8, 8), 1, 260, True),      # two blocks of lower bands
