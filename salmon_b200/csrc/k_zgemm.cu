@@ -292,14 +292,15 @@ constexpr double GS_PIVOT = 1e-9, GS_ONCE = 2.0, GS_COND = 1e11;
 
 // Sums the panel's Gram matrix, factors it and writes Z[k][n][m] = (L^-H)(m, n):
 // one CTA per k-point, thread (i, l) owns element (i, l) of the trailing matrix and
-// of L^-1 (eliminated together, one barrier a column).
+// of L^-1 (eliminated together, one barrier a column).  bad[k]: refused, the panel must not
+// be multiplied (0 times an infinity would spread it over the panel); skip[k]: no second round.
 __global__ void __launch_bounds__(GSP* GSP) k_gs_chol(const double2* __restrict__ part, int nsplit, int nkl, int pb,
                                                       double Hxyz, int round, int* __restrict__ bad,
-                                                      int* __restrict__ once, double2* __restrict__ Z) {
+                                                      int* __restrict__ skip, double2* __restrict__ Z) {
   __shared__ double2 A[GSP][GSP + 1], W[GSP][GSP + 1];
   __shared__ double d0[GSP], inv[GSP], sh[32];
   const int k = blockIdx.x, i = threadIdx.x / GSP, l = threadIdx.x % GSP;
-  if (round == 1 && once[k]) return;  // (the products of this round return too)
+  if (round == 1 && skip[k]) return;  // (the products of this round return too)
   double2 a = make_double2(0.0, 0.0);
   if (i < pb && l <= i)
     for (int sp = 0; sp < nsplit; ++sp) {
@@ -311,7 +312,7 @@ __global__ void __launch_bounds__(GSP* GSP) k_gs_chol(const double2* __restrict_
   A[i][l] = a;
   W[i][l] = make_double2(i == l ? 1.0 : 0.0, 0.0);
   if (i == l) d0[i] = a.x;
-  bool ok = round == 0 || bad[k] == 0;
+  bool ok = true;
   for (int j = 0; j < pb && ok; ++j) {
     __syncthreads();
     const double d = A[j][j].x;
@@ -335,18 +336,12 @@ __global__ void __launch_bounds__(GSP* GSP) k_gs_chol(const double2* __restrict_
   block_allsum<1>(tau, sh);
   const bool good = tau[0] <= GS_ONCE * pb;  // the same in every thread; false for NaN
   ok = ok && (good || (round == 0 && tau[0] <= GS_COND));
-  if (i < pb && l < pb) {
-    double2 z = make_double2(i == l ? 1.0 : 0.0, 0.0);  // a refused panel: left as it is
-    if (ok) z = l <= i ? make_double2(W[i][l].x * inv[i], -W[i][l].y * inv[i]) : make_double2(0.0, 0.0);
-    Z[((size_t)k * GSP + i) * GSP + l] = z;
-  }
+  if (ok && i < pb && l < pb)
+    Z[((size_t)k * GSP + i) * GSP + l] =
+        l <= i ? make_double2(W[i][l].x * inv[i], -W[i][l].y * inv[i]) : make_double2(0.0, 0.0);
   if (threadIdx.x == 0) {
-    if (round == 0) {
-      bad[k] = ok ? 0 : 1;
-      once[k] = ok && good ? 1 : 0;
-    } else if (!ok) {
-      bad[k] = 1;
-    }
+    bad[k] = !ok;
+    if (round == 0 || !ok) skip[k] = !ok || good;
   }
 }
 
@@ -371,14 +366,15 @@ cudaError_t launch_gram_schmidt(const System& s, double2* zu) {
     const int pb = std::min(pw, s.NB - p0), rest = s.NB - p0 - pb;
     double2* P = zu + (size_t)p0 * s.NL;
     int ns = 1;
-    int* once = s.gs_bad + s.nkl;
+    int* skip = s.gs_bad + s.nkl;
     for (int round = 0; round < 2; ++round) {
-      const int* skip = round ? once : nullptr;
-      if ((e = launch_hn(s, P, pb, P, pb, true, s.gs_part, ns, skip)) != cudaSuccess) return e;
-      k_gs_chol<<<s.nkl, GSP * GSP, 0, s.launch_stream()>>>(s.gs_part, ns, s.nkl, pb, s.Hxyz, round, s.gs_bad, once,
+      if ((e = launch_hn(s, P, pb, P, pb, true, s.gs_part, ns, round ? skip : nullptr)) != cudaSuccess) return e;
+      k_gs_chol<<<s.nkl, GSP * GSP, 0, s.launch_stream()>>>(s.gs_part, ns, s.nkl, pb, s.Hxyz, round, s.gs_bad, skip,
                                                             s.gs_R);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
-      if ((e = launch_nn(s, P, pb, s.gs_R, (size_t)GSP * GSP, GSP, pb, nullptr, P, skip)) != cudaSuccess) return e;
+      if ((e = launch_nn(s, P, pb, s.gs_R, (size_t)GSP * GSP, GSP, pb, nullptr, P, round ? skip : s.gs_bad)) !=
+          cudaSuccess)
+        return e;
     }
     if ((e = launch_gram_schmidt_panel(s, zu, p0, pb, s.gs_bad)) != cudaSuccess) return e;
     if (rest > 0) {

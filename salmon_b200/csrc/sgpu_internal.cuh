@@ -186,7 +186,7 @@ struct System {
   double2* gs_part = nullptr;      // [gs_part_elems] partial products of the split-K kernels
   size_t gs_part_elems = 0;
   double2* gs_R = nullptr;         // [nkl][32][32] inverse Cholesky factor of a Gram-Schmidt panel
-  int* gs_bad = nullptr;           // [nkl] panels left to the one-by-one Gram-Schmidt, [nkl] panels done in one round
+  int* gs_bad = nullptr;           // [nkl] panels left to the one-by-one Gram-Schmidt, [nkl] panels without a second round
   double2* gs_M = nullptr;         // [nkl][NB][256] rows of (I + L)^-1, L the lower bands' overlaps (k_gs.cu)
   double* gs_MR = nullptr;         // [nkl][NB][256] the same for the overlaps' real parts
   double2* gs_dots = nullptr;      // [nkl][CG_DOT_SPLITS][256] partial inner products with the lower bands

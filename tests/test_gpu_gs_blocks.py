@@ -99,6 +99,21 @@ def test_gram_schmidt_second_round(cuda_lib, eps):
     assert rel(out, O.gram_schmidt(sysm, z)) < 1e-14 / eps + 1e-13
 
 
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("band", [0, 17, 38])
+def test_gram_schmidt_non_finite_band(cuda_lib, band, value):
+    """The bands below a non-finite one stay what they are without it, as one by one."""
+    sysm, kAc, vloc, z = raw_system((7, 9, 11), 2, 40)
+    z[1, band, 100] = value
+    with np.errstate(all="ignore"):
+        ref = O.gram_schmidt(sysm, z)
+    out = gram_schmidt(sysm, kAc, vloc, z)
+    assert rel(out[0], ref[0]) < 1e-12
+    assert np.isnan(out[1, band:]).any(axis=1).all()
+    if band:
+        assert rel(out[1, :band], ref[1, :band]) < 1e-12
+
+
 @pytest.mark.parametrize("grid,nk,nb,orthonormal", [
     ((7, 9, 11), 2, 9, False),      # bands not orthogonal: the order of the projections counts
     ((8, 8, 8), 1, 260, True),      # two blocks of lower bands
