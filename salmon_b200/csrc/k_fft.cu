@@ -362,14 +362,9 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft_mid_tpa(double2* z, TpaArgs
   });
 }
 
-template <typename K>
-static cudaError_t fft_smem_limit(K kern, size_t smem) {
-  return smem > 48 * 1024 ? raise_smem_limit((const void*)kern, smem) : cudaSuccess;
-}
-
 static cudaError_t launch_fft_planes(const System& s, const double* real, double2* z, int nvec, int sign) {
   const size_t smem = fft_plane_smem(s);
-  const cudaError_t e = real ? fft_smem_limit(k_fft_planes<true>, smem) : fft_smem_limit(k_fft_planes<false>, smem);
+  const cudaError_t e = raise_smem_limit(real ? (const void*)k_fft_planes<true> : (const void*)k_fft_planes<false>, smem);
   if (e != cudaSuccess) return e;
   const dim3 grid(s.NLx, nvec);
   if (real) k_fft_planes<true><<<grid, FFP_THREADS, smem, s.launch_stream()>>>(real, z, s.NLx, s.NLy, s.NLz, sign, 1.0);
@@ -474,7 +469,7 @@ __global__ void __launch_bounds__(FFP_THREADS) k_fft_planes_vloc(const double2* 
 cudaError_t launch_fft_planes_vloc(const System& s, const double2* z, const double* rho, double* part,
                                    double* energies_dev) {
   const size_t smem = fft_plane_smem(s);
-  const cudaError_t e = fft_smem_limit(k_fft_planes_vloc, smem);
+  const cudaError_t e = raise_smem_limit((const void*)k_fft_planes_vloc, smem);
   if (e != cudaSuccess) return e;
   k_fft_planes_vloc<<<s.NLx, FFP_THREADS, smem, s.launch_stream()>>>(z, s.NLx, s.NLy, s.NLz, rho, s.vpsl, s.vloc64,
                                                                      s.vloc32, part, s.Hxyz, s.xc_count, energies_dev);

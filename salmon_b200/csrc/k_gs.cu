@@ -985,10 +985,8 @@ cudaError_t launch_jacobi(const System& s, double2* A, double2* V, int max_sweep
   const size_t base = jac_pair_bytes(s.NB) + 16, both = 2 * (size_t)s.NB * s.NB * sizeof(double2);
   const int in_smem = base + both <= JAC_SMEM;
   const size_t smem = base + (in_smem ? both : 0);
-  if (smem > 48 * 1024) {
-    const cudaError_t e = raise_smem_limit((const void*)k_jacobi_herm, smem);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t e = raise_smem_limit((const void*)k_jacobi_herm, smem);
+  if (e != cudaSuccess) return e;
   const int nt = 32 * std::min(32, std::max(8, (s.NB + 1) / 2 + 1));  // a warp per column pair, and one for the rotations
   k_jacobi_herm<<<s.nkl, nt, smem, s.launch_stream()>>>(A, V, s.NB, max_sweeps, in_smem, w, sweeps);
   return cudaGetLastError();

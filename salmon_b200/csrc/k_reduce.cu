@@ -281,10 +281,8 @@ static cudaError_t fwd_march(System& s, double* out, int& nx) {
   nx = march_blocks(s.NLy, s.NLz);
   const int nt = (GB / 2 * s.NLz + 31) / 32 * 32;
   const size_t smem = 2 * (size_t)(GB + 4) * s.NLz * sizeof(double2);
-  if (smem > 48 * 1024) {
-    const cudaError_t e = raise_smem_limit((const void*)k_fwd_march<R, EKIN>, smem);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t e = raise_smem_limit((const void*)k_fwd_march<R, EKIN>, smem);
+  if (e != cudaSuccess) return e;
   k_fwd_march<R, EKIN><<<s.norb * nx, nt, smem, s.launch_stream()>>>((const C2<R>*)s.zu, s.NLx, s.NLy, s.NLz, GB, nx,
                                                                      s.NBocc, s.kAc_d, c, out);
   return cudaGetLastError();

@@ -303,15 +303,21 @@ int pass2_rows(int prec, int NLy, int NLz);
 // launch (needed before capturing its launches into a graph).
 cudaError_t prepare_pass(const System& s);
 cudaError_t prepare_kb(const System& s);
-// Raises a kernel's dynamic shared-memory limit to at least `bytes` (never
-// lowers it, so handles of different sizes sharing a kernel keep working).
+// Lets a kernel launch with `bytes` of dynamic shared memory: raises its limit where the
+// dynamic and the static part together exceed the default of 48 KB (never lowers it, so
+// handles of different sizes sharing a kernel keep working).  No kernel has more than
+// SMEM_STATIC bytes of static shared memory, so small sizes return without a query.
+constexpr size_t SMEM_DEFAULT = 48 * 1024, SMEM_STATIC = 12 * 1024;
 inline cudaError_t raise_smem_limit(const void* func, size_t bytes) {
+  if (bytes + SMEM_STATIC <= SMEM_DEFAULT) return cudaSuccess;
   cudaFuncAttributes fa;
   cudaError_t e = cudaFuncGetAttributes(&fa, func);
   if (e != cudaSuccess) return e;
-  if ((size_t)fa.maxDynamicSharedSizeBytes >= bytes) return cudaSuccess;
-  return cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}  // shared-memory attribute of the KB tile kernel
+  const size_t now = (size_t)fa.maxDynamicSharedSizeBytes;
+  if (bytes + fa.sharedSizeBytes <= SMEM_DEFAULT || (bytes <= now && now > SMEM_DEFAULT)) return cudaSuccess;
+  return cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes > now ? bytes : now));
+}
+  // shared-memory attribute of the KB tile kernel
 bool kb_tile_fits(const System& s);
 int pass_block_threads(int NLy, int NLz);
 
