@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(GY / NP * GZ) k_current_march_yh(const C2<R>* 
 #pragma unroll
   for (int n = 1; n <= 4; ++n) zo[n - 1] = yl * GZ + ((z + n) % GZ);
   // register queue: at phase P (plane x = 5i + P) plane x+m sits in q[(P+m) % 5];
-  // the march is unrolled five times so the queue rotates by renaming (NLx >= 6)
+  // the march is unrolled five times so the queue rotates by renaming (NLx >= 5)
   double2 q[5];
 #pragma unroll
   for (int m = 0; m < 5; ++m) q[m] = to_d2(__ldg(E + (size_t)m * NYZ + own));
@@ -681,7 +681,10 @@ static cudaError_t current_stencil(System& s, const Nab12& nab, double* part, in
   // At 32^3 x 2048 orbitals, complex(4): 0.328 against 0.388 ms; two rows per
   // thread at 118 registers (two CTAs per SM) 0.709 ms, one CTA per plane 0.344 ms
   // (complex(8): 0.394 / 0.403 / 0.642 / 0.423 ms)
-  if (s.cur_fixed && s.NLy == 32 && s.NLz == 32) {
+  // Both fixed forms fill their queue with planes 0 .. 4 as they lie in memory; grids of
+  // fewer planes take the march for any shape, which wraps them.
+  const bool fixed = s.cur_fixed && s.NLx >= 5;
+  if (fixed && s.NLy == 32 && s.NLz == 32) {
     if (s.cur_fixed == 2) {
       nx = 4;
       return current_march_yh<R, 32, 32, 4>(s, nab, part);
@@ -692,7 +695,7 @@ static cudaError_t current_stencil(System& s, const Nab12& nab, double* part, in
   // 48x48 planes (the 48^3 grid): six CTAs of 8 rows per orbital plane (two rows per
   // thread, 192 threads; value 2: one row per thread, 384 threads): 0.284 against
   // 0.313 ms at 432 orbitals, complex(4); 0.298 against 0.328 ms complex(8)
-  if (s.cur_fixed && s.NLy == 48 && s.NLz == 48) {
+  if (fixed && s.NLy == 48 && s.NLz == 48) {
     nx = 6;
     return s.cur_fixed == 2 ? current_march_yh<R, 48, 48, 6>(s, nab, part) : current_march_y2<R, 48, 48, 6>(s, nab, part);
   }

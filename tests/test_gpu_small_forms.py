@@ -82,6 +82,26 @@ def test_current_and_energy_march(cuda_lib, precision, shape):
 
 
 @pytest.mark.parametrize("precision", ["c128", "c64"])
+@pytest.mark.parametrize("cur_fixed", [1, 2])
+@pytest.mark.parametrize("shape", [(1, 32, 32), (3, 32, 32), (4, 48, 48), (5, 32, 32), (6, 48, 48)])
+def test_current_of_few_planes(cuda_lib, precision, cur_fixed, shape):
+    """Planes with a fixed form of the current: around the length of its queue (five planes),
+    as a call of its own and out of a step that computes the sums beside the update."""
+    from salmon_b200.rt import GpuSystem
+    sysm, kAc, vloc, zu = S.small_system(*shape, nk=1, nb=3, a=(shape[0] * 0.5, 9.0, 9.5), seed=5)
+    z = zu if precision == "c128" else zu.astype(np.complex64).astype(np.complex128)
+    with GpuSystem(sysm, precision) as g:
+        g.set_param("cur_fixed", cur_fixed)
+        g.set_state(zu)
+        g.set_vloc(vloc)
+        assert rel(g.current_RT(kAc), O.current(sysm, kAc, z)) < 1e-11
+        g.update_projector(kAc)
+        g.hamiltonian(0.004, flag_current=True)
+        z1 = np.asarray(g.get_state(), np.complex128)
+        assert rel(g.current_RT(kAc), O.current(sysm, kAc, z1)) < 1e-11
+
+
+@pytest.mark.parametrize("precision", ["c128", "c64"])
 @pytest.mark.parametrize("shape,nslab", [((3, 32, 32), 1), ((10, 32, 32), 3), ((7, 48, 48), 2), ((5, 16, 32), 1),
                                          ((4, 16, 16), 1)])
 def test_two_row_pass(cuda_lib, precision, shape, nslab):
