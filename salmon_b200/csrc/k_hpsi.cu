@@ -923,10 +923,13 @@ bool kb_tile_fits(const System& s) {  // dynamic + static shared memory of both 
 }
 
 cudaError_t prepare_kb(const System& s) {
-  cudaError_t e = raise_smem_limit((const void*)k_kb_tile<float>, KbtGeom<float>::smem(s.Nps));
-  if (e == cudaSuccess) e = raise_smem_limit((const void*)k_kb_tile<double>, KbtGeom<double>::smem(s.Nps));
-  if (e == cudaSuccess) e = raise_smem_limit((const void*)k_kb_tile<float, true>, KbtGeom<float>::smem(s.Nps));
-  if (e == cudaSuccess) e = raise_smem_limit((const void*)k_kb_tile<double, true>, KbtGeom<double>::smem(s.Nps));
+  cudaError_t e = cudaSuccess;
+  if (kb_tile_fits(s)) {  // (the tile kernels hold tables of Nps entries, whatever the atoms use of them)
+    e = raise_smem_limit((const void*)k_kb_tile<float>, KbtGeom<float>::smem(s.Nps));
+    if (e == cudaSuccess) e = raise_smem_limit((const void*)k_kb_tile<double>, KbtGeom<double>::smem(s.Nps));
+    if (e == cudaSuccess) e = raise_smem_limit((const void*)k_kb_tile<float, true>, KbtGeom<float>::smem(s.Nps));
+    if (e == cudaSuccess) e = raise_smem_limit((const void*)k_kb_tile<double, true>, KbtGeom<double>::smem(s.Nps));
+  }
   if (kb_atom_fits(s)) {
     if (e == cudaSuccess) e = raise_smem_limit((const void*)k_kb_atom<float>, KbaGeom<float>::smem(s.max_mps));
     if (e == cudaSuccess) e = raise_smem_limit((const void*)k_kb_atom<double>, KbaGeom<double>::smem(s.max_mps));

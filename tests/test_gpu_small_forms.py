@@ -138,3 +138,32 @@ def test_whole_atom_projections(cuda_lib, precision, nb, rps):
         g.update_projector(kAc)
         g.hamiltonian(0.02)
         assert rel(g.get_state(), O.hamiltonian(sysm, kAc, vloc, zproj, 0.02, z_in)) < TOL[precision]
+
+
+@pytest.mark.parametrize("precision", ["c128", "c64"])
+def test_projector_tables_wider_than_the_atoms(cuda_lib, precision):
+    """Atoms of few points in tables with room for 30000: the tile kernels do not fit in shared
+    memory, the whole-atom form does; a single step and a captured one."""
+    from salmon_b200.rt import GpuBatch, GpuSystem
+    sysm, kAc, vloc, zu = S.small_system(8, 10, 12, nk=2, nb=5, seed=9)
+    _, zproj = O.update_projector(sysm, kAc)
+    z_in = zu if precision == "c128" else zu.astype(np.complex64).astype(np.complex128)
+    ref = O.hamiltonian(sysm, kAc, vloc, zproj, 0.02, z_in)
+    n = sysm.uV.shape[1]
+    for name in ("Jxyz", "Jxx", "Jyy", "Jzz", "uV"):
+        t = getattr(sysm, name)
+        wide = np.zeros((t.shape[0], 30000), t.dtype)
+        wide[:, :n] = t
+        setattr(sysm, name, wide)
+    with GpuSystem(sysm, precision) as g:
+        g.set_param("taylor_kernel", 1)
+        g.set_vloc(vloc)
+        g.update_projector(kAc)
+        g.set_state(zu)
+        g.hamiltonian(0.02)
+        assert rel(g.get_state(), ref) < TOL[precision]
+        g.set_state(zu)
+        b = GpuBatch([g])
+        b.step([0.02])
+        assert rel(g.get_state(), ref) < TOL[precision]
+        b.close()
