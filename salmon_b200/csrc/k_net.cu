@@ -299,7 +299,7 @@ template <int CI, int CO>
 static cudaError_t conv_bwd_w(System& s, NetState& ns, const float* gout, const bf16* in, float* dW, int nvec) {
   const NetGeom G = geom(s);
   const size_t smem = (size_t)s.NLy * s.NLz * (3 * CI * sizeof(bf16) + CO * sizeof(float));
-  cudaError_t e = cudaFuncSetAttribute(k_conv_bwd_w<CI, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = raise_smem_limit((const void*)k_conv_bwd_w<CI, CO>, smem);
   if (e != cudaSuccess) return e;
   k_conv_bwd_w<CI, CO><<<dim3(s.NLx, nvec), 256, smem, s.launch_stream()>>>(gout, in, ns.part, G);
   const int nw = CO * CI * NTAP;

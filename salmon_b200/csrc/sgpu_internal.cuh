@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -305,11 +306,14 @@ cudaError_t prepare_pass(const System& s);
 cudaError_t prepare_kb(const System& s);
 // Lets a kernel launch with `bytes` of dynamic shared memory: raises its limit where the
 // dynamic and the static part together exceed the default of 48 KB (never lowers it, so
-// handles of different sizes sharing a kernel keep working).  No kernel has more than
+// handles of different sizes sharing a kernel keep working, also from several host threads:
+// the query and the change are one step under the lock).  No kernel has more than
 // SMEM_STATIC bytes of static shared memory, so small sizes return without a query.
 constexpr size_t SMEM_DEFAULT = 48 * 1024, SMEM_STATIC = 12 * 1024;
+inline std::mutex smem_limit_lock;
 inline cudaError_t raise_smem_limit(const void* func, size_t bytes) {
   if (bytes + SMEM_STATIC <= SMEM_DEFAULT) return cudaSuccess;
+  std::lock_guard<std::mutex> guard(smem_limit_lock);
   cudaFuncAttributes fa;
   cudaError_t e = cudaFuncGetAttributes(&fa, func);
   if (e != cudaSuccess) return e;

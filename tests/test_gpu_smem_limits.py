@@ -1,6 +1,7 @@
 """Sizes whose dynamic shared memory alone stays below the default limit of 48 KB and passes
 it together with the kernel's static part.  A limit raised by an earlier, larger grid would
-hide a missing one, so each case runs in its own process.
+hide a missing one, so each case runs in its own process.  So does the first use of one kernel
+by several threads at once.
 
 Tolerances: FP64 sums in another order, 1e-12 (potential), 1e-11 (current, energies,
 eigenvalues), as for the other sizes."""
@@ -57,7 +58,27 @@ def eigensolver(*shape):
     assert rel(esp, O.diag(sysm, kAc, vloc, z)[1]) < 1e-11
 
 
-@pytest.mark.parametrize("what,shape", [("potential", (2, 27, 54)), ("potential", (3, 18, 81)), ("march", (3, 2, 252)),
+def threads(*rows):
+    """Handles whose planes differ in size, first used at the same moment by a thread each."""
+    from concurrent.futures import ThreadPoolExecutor
+    from threading import Barrier
+    from salmon_b200.rt import GpuSystem
+    start = Barrier(len(rows))
+
+    def one(n):
+        sysm = grid_system((2, n, 96))
+        with GpuSystem(sysm) as g:
+            g.set_vpsl(np.zeros(sysm.NL))
+            start.wait()
+            for _ in range(20):
+                g.update_vloc(np.ones(sysm.NL))
+
+    with ThreadPoolExecutor(len(rows)) as ex:
+        list(ex.map(one, rows))
+
+
+@pytest.mark.parametrize("what,shape", [("threads", (16, 24, 27, 32, 36, 48, 54, 64)),
+                                        ("potential", (2, 27, 54)), ("potential", (3, 18, 81)), ("march", (3, 2, 252)),
                                         ("march", (6, 4, 256)), ("eigensolver", (9, 10, 10))])
 def test_default_limit_edge(cuda_lib, what, shape):
     here = os.path.dirname(os.path.abspath(__file__))
