@@ -25,7 +25,6 @@ constexpr int GS_THREADS = 512;
 namespace cgx = cooperative_groups;
 
 constexpr int GRP_NV = 8;    // values of one sum
-constexpr int CGB = 256;     // lower bands projected out together (grp_project)
 
 struct GrpShared {
   double sh[32 * GRP_NV];

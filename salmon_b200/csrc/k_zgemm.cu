@@ -287,7 +287,7 @@ cudaError_t launch_rotate(const System& s, const double2* in, const double2* Z, 
 // |<u_i|u_j> - delta_ij|, 32 bands with a sine of 0.51 / 0.6 / 0.8 to the band before: one by
 // one 1e-8 / 3e-12 / 2e-15, here 1e-8 (one by one) / 6e-16 (two rounds) / 9e-16.
 // One Gram-Schmidt at 16x16x32, 32 k, 40 bands: 3.56 -> 0.5 ms.
-constexpr int GSP = 32;  // bands of a panel, = the output tile of k_zgemm_nn (in place)
+static_assert(GSP == ZT, "a panel is one output tile of k_zgemm_nn (in place)");
 constexpr double GS_PIVOT = 1e-9, GS_ONCE = 2.0, GS_COND = 1e11;
 
 // Sums the panel's Gram matrix, factors it and writes Z[k][n][m] = (L^-H)(m, n):

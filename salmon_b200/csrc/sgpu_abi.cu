@@ -54,6 +54,23 @@ void free_state_buffers(System* s) {
   s->zu = nullptr;
 }
 
+// every device buffer of the ground state
+std::vector<void**> gs_buffers(System* s) {
+  return {(void**)&s->gs_zu,  (void**)&s->gs_aux,    (void**)&s->gs_W,   (void**)&s->gs_st,   (void**)&s->gs_part,
+          (void**)&s->gs_A,   (void**)&s->gs_V,      (void**)&s->gs_w,   (void**)&s->gs_R,    (void**)&s->gs_bad,
+          (void**)&s->gs_M,   (void**)&s->gs_MR,     (void**)&s->gs_dots, (void**)&s->gs_iters, (void**)&s->gs_sweeps,
+          (void**)&s->gs_out, (void**)&s->gs_res,    (void**)&s->gs_tb,  (void**)&s->occ_gs};
+}
+
+void gs_free(System* s) {
+  for (void** p : gs_buffers(s)) {
+    cudaFree(*p);
+    *p = nullptr;
+  }
+  if (s->gs_h) cudaFreeHost(s->gs_h);
+  s->gs_h = nullptr;
+}
+
 int alloc_state_buffers(System* s) {
   ++s->gen;
   const size_t n = (size_t)s->norb * s->NL;
@@ -540,11 +557,9 @@ int sgpu_destroy(sgpu_handle h) {
                   s->lma_list, s->iuV_d, s->lma_atom, s->uV_d, s->zproj64, s->zproj32, s->sp_off, s->rec, s->cont, s->qmap, s->kbq, s->kb_multi, s->lqi, s->Sbuf, s->Wbuf,
                   s->U, s->Up, s->Uw, s->red, s->stage, s->cur_part};
   for (void* p : bufs) cudaFree(p);
-  void* gbufs[] = {s->gs_zu, s->gs_aux, s->gs_W, s->gs_st, s->gs_part, s->gs_A, s->gs_V, s->gs_w, s->gs_sweeps,
-                   s->occ_gs, s->p2_blk[0], s->p2_blk[1], s->gs_out, s->gs_R, s->gs_bad, s->gs_M, s->gs_MR, s->gs_dots, s->gs_iters, s->gs_res, s->gs_tb, s->vpsl, s->rho_d, s->exc_d, s->sp_blk,
-                   s->vloc_hist};
+  gs_free(s);
+  void* gbufs[] = {s->p2_blk[0], s->p2_blk[1], s->vpsl, s->rho_d, s->exc_d, s->sp_blk, s->vloc_hist};
   for (void* p : gbufs) cudaFree(p);
-  if (s->gs_h) cudaFreeHost(s->gs_h);
   if (s->red_h) cudaFreeHost(s->red_h);
   if (s->aux) cudaStreamSynchronize(s->aux);
   if (s->in_h) cudaFreeHost(s->in_h);
@@ -856,8 +871,27 @@ int sgpu_time_kernel(sgpu_handle h, int kernel, int reps, double* ms_per_launch)
 // ------------------------------------------------------------ ground state --
 namespace {
 
-int gs_alloc(System* s) {
-  if (s->gs_zu) return 0;
+// A buffer of `rows` rows of `row_bytes` grown to `want` rows; on failure it keeps its old size.
+int grow_rows(System* s, void** p, size_t& rows, size_t want, size_t row_bytes) {
+  if (want <= rows) return 0;
+  CK(cudaStreamSynchronize(s->stream));
+  cudaFree(*p);
+  *p = nullptr;
+  const cudaError_t e = cudaMalloc(p, want * row_bytes);
+  if (e == cudaSuccess) {
+    rows = want;
+    return 0;
+  }
+  (void)cudaGetLastError();
+  if (cudaMalloc(p, rows * row_bytes) != cudaSuccess) {  // (just freed; without it no H application may run)
+    (void)cudaGetLastError();
+    rows = 0;
+    s->have_proj = false;
+  }
+  return cuda_fail(e, "ground-state buffers");
+}
+
+int gs_alloc_all(System* s) {
   const size_t nbl = (size_t)s->nkl * s->NB * s->NL;
   // partial products of the split-K kernels: about four 32 x 32 tiles per SM
   const size_t nt = (s->NB + 31) / 32, nn = (size_t)s->nkl * s->NB * s->NB;
@@ -871,11 +905,11 @@ int gs_alloc(System* s) {
   CK(cudaMalloc(&s->gs_A, (size_t)s->nkl * s->NB * s->NB * sizeof(double2)));
   CK(cudaMalloc(&s->gs_V, (size_t)s->nkl * s->NB * s->NB * sizeof(double2)));
   CK(cudaMalloc(&s->gs_w, (size_t)s->nkl * s->NB * sizeof(double)));
-  CK(cudaMalloc(&s->gs_R, (size_t)s->nkl * 32 * 32 * sizeof(double2)));
+  CK(cudaMalloc(&s->gs_R, (size_t)s->nkl * sgpu::GSP * sgpu::GSP * sizeof(double2)));
   CK(cudaMalloc(&s->gs_bad, 2 * (size_t)s->nkl * sizeof(int)));
-  CK(cudaMalloc(&s->gs_M, (size_t)s->nkl * s->NB * 256 * sizeof(double2)));
-  CK(cudaMalloc(&s->gs_MR, (size_t)s->nkl * s->NB * 256 * sizeof(double)));
-  CK(cudaMalloc(&s->gs_dots, (size_t)s->nkl * sgpu::CG_DOT_SPLITS * 256 * sizeof(double2)));
+  CK(cudaMalloc(&s->gs_M, (size_t)s->nkl * s->NB * sgpu::CGB * sizeof(double2)));
+  CK(cudaMalloc(&s->gs_MR, (size_t)s->nkl * s->NB * sgpu::CGB * sizeof(double)));
+  CK(cudaMalloc(&s->gs_dots, (size_t)s->nkl * sgpu::CG_DOT_SPLITS * sgpu::CGB * sizeof(double2)));
   CK(cudaMalloc(&s->gs_iters, (size_t)s->nkl * s->NB * sizeof(int)));
   CK(cudaMalloc(&s->gs_sweeps, (size_t)s->nkl * sizeof(int)));
   CK(cudaMalloc(&s->gs_out, (size_t)s->nkl * s->NB * sizeof(double)));
@@ -888,29 +922,26 @@ int gs_alloc(System* s) {
     for (int b = 0; b < s->NB; ++b) occ[(size_t)kl * s->NB + b] = s->occ_h[(size_t)(s->NK_s - 1 + kl) * s->NB + b];
   CK(cudaMalloc(&s->occ_gs, occ.size() * sizeof(double)));
   CK(cudaMemcpyAsync(s->occ_gs, occ.data(), occ.size() * sizeof(double), cudaMemcpyHostToDevice, s->stream));
+  CK(cudaStreamSynchronize(s->stream));  // (the copy reads occ)
   const size_t rows = std::max((size_t)s->norb, (size_t)s->nkl * s->NB);
-  if (rows > s->W_rows) {
-    CK(cudaStreamSynchronize(s->stream));
-    cudaFree(s->Wbuf);
-    s->Wbuf = nullptr;
-    CK(cudaMalloc(&s->Wbuf, rows * std::max(1, s->nsp) * sizeof(double2)));
-    s->W_rows = rows;
+  const size_t u_bytes = std::max(1, s->Nlma) * sizeof(double2);
+  if (int rc = grow_rows(s, (void**)&s->Wbuf, s->W_rows, rows, std::max(1, s->nsp) * sizeof(double2))) return rc;
+  if (int rc = grow_rows(s, (void**)&s->U, s->U_rows, rows, u_bytes)) return rc;
+  // the split KB form's partial projections
+  return grow_rows(s, (void**)&s->Up, s->Up_rows, sgpu::KB_USPLIT_MAX * rows, u_bytes);
+}
+
+// All of the ground state's buffers, or none: the next call tries again.
+int gs_alloc(System* s) {
+  if (s->gs_alloc_done) return 0;
+  const int rc = gs_alloc_all(s);
+  if (rc) {
+    cudaStreamSynchronize(s->stream);
+    gs_free(s);
+    (void)cudaGetLastError();
+    return rc;
   }
-  if (rows > s->U_rows) {
-    CK(cudaStreamSynchronize(s->stream));
-    cudaFree(s->U);
-    s->U = nullptr;
-    CK(cudaMalloc(&s->U, rows * std::max(1, s->Nlma) * sizeof(double2)));
-    s->U_rows = rows;
-  }
-  if ((size_t)sgpu::KB_USPLIT_MAX * rows > s->Up_rows) {  // the split KB form's partial projections
-    CK(cudaStreamSynchronize(s->stream));
-    cudaFree(s->Up);
-    s->Up = nullptr;
-    CK(cudaMalloc(&s->Up, (size_t)sgpu::KB_USPLIT_MAX * rows * std::max(1, s->Nlma) * sizeof(double2)));
-    s->Up_rows = (size_t)sgpu::KB_USPLIT_MAX * rows;
-  }
-  CK(cudaStreamSynchronize(s->stream));
+  s->gs_alloc_done = true;
   return 0;
 }
 

@@ -13,6 +13,8 @@
 namespace sgpu {
 
 constexpr int KB_USPLIT_MAX = 8;  // point ranges of the split KB projections
+constexpr int CGB = 256;          // lower bands that CG projects out together
+constexpr int GSP = 32;           // bands of a Gram-Schmidt panel
 
 // ---------------------------------------------------------------- complex --
 template <typename R> struct C2Of;
@@ -186,11 +188,11 @@ struct System {
   void* gs_st = nullptr;           // [nkl] CG state
   double2* gs_part = nullptr;      // [gs_part_elems] partial products of the split-K kernels
   size_t gs_part_elems = 0;
-  double2* gs_R = nullptr;         // [nkl][32][32] inverse Cholesky factor of a Gram-Schmidt panel
+  double2* gs_R = nullptr;         // [nkl][GSP][GSP] inverse Cholesky factor of a Gram-Schmidt panel
   int* gs_bad = nullptr;           // [nkl] panels left to the one-by-one Gram-Schmidt, [nkl] panels without a second round
-  double2* gs_M = nullptr;         // [nkl][NB][256] rows of (I + L)^-1, L the lower bands' overlaps (k_gs.cu)
-  double* gs_MR = nullptr;         // [nkl][NB][256] the same for the overlaps' real parts
-  double2* gs_dots = nullptr;      // [nkl][CG_DOT_SPLITS][256] partial inner products with the lower bands
+  double2* gs_M = nullptr;         // [nkl][NB][CGB] rows of (I + L)^-1, L the lower bands' overlaps (k_gs.cu)
+  double* gs_MR = nullptr;         // [nkl][NB][CGB] the same for the overlaps' real parts
+  double2* gs_dots = nullptr;      // [nkl][CG_DOT_SPLITS][CGB] partial inner products with the lower bands
   int* gs_iters = nullptr;         // [nkl][NB] CG iterations of each band
   double2* gs_A = nullptr;         // [nkl][NB][NB]
   double2* gs_V = nullptr;         // [nkl][NB][NB]
@@ -199,6 +201,7 @@ struct System {
   double* occ_gs = nullptr;        // [nkl][NB]
   double* gs_out = nullptr;        // [nkl][NB] device results
   double* gs_h = nullptr;          // pinned host staging [nkl][NB]
+  bool gs_alloc_done = false;      // every buffer above is there
   bool have_gs = false;
   size_t U_rows = 0;               // orbitals U can hold
 
