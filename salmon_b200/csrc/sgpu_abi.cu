@@ -872,8 +872,10 @@ int sgpu_time_kernel(sgpu_handle h, int kernel, int reps, double* ms_per_launch)
 namespace {
 
 // A buffer of `rows` rows of `row_bytes` grown to `want` rows; on failure it keeps its old size.
+// Captured steps hold its address: they are captured again.
 int grow_rows(System* s, void** p, size_t& rows, size_t want, size_t row_bytes) {
   if (want <= rows) return 0;
+  ++s->gen;
   CK(cudaStreamSynchronize(s->stream));
   cudaFree(*p);
   *p = nullptr;

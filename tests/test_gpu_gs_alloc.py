@@ -29,3 +29,26 @@ def test_out_of_memory(cuda_lib):
         g.set_state(zu)
         g.hamiltonian(0.02)
         assert rel(g.get_state(), ref) < 1e-12
+
+
+@pytest.mark.parametrize("grid", [(8, 10, 12), (16, 16, 16)])
+def test_captured_step_after_growth(cuda_lib, grid):
+    """More bands in the ground state than in real time: the projections' buffers grow, and a
+    batch that captured a step before is captured anew."""
+    from salmon_b200.rt import GpuBatch, GpuSystem
+    sysm, kAc, vloc, zu = S.small_system(*grid, nk=2, nb=40, seed=2)
+    sysm.NBoccmax = 3
+    zu = np.ascontiguousarray(zu[:, :3])
+    _, zproj = O.update_projector(sysm, kAc)
+    one = O.hamiltonian(sysm, kAc, vloc, zproj, 0.02, zu)
+    two = O.hamiltonian(sysm, kAc, vloc, zproj, 0.02, one)
+    with GpuSystem(sysm) as g:
+        g.set_vloc(vloc)
+        g.update_projector(kAc)
+        g.set_state(zu)
+        with GpuBatch([g]) as b:
+            b.step(0.02)
+            assert rel(g.get_state(), one) < 1e-12
+            g.gs_set_state(np.ones((2, 40, sysm.NL), complex))
+            b.step(0.02)
+            assert rel(g.get_state(), two) < 1e-12
