@@ -841,15 +841,19 @@ struct JacPair {
 
 constexpr size_t JAC_SMEM = 220 * 1024;
 
-static size_t jac_pair_bytes(int NB) { return 2 * (size_t)((NB + 1) / 2) * sizeof(JacPair) + (size_t)NB * (sizeof(double) + sizeof(int)); }
+// the rotations of two steps; the eigenvalues and their order.  Beyond 3700 bands the
+// rotations too are in global memory (gpr).
+static size_t jac_pair_bytes(int NB) { return 2 * (size_t)((NB + 1) / 2) * sizeof(JacPair); }
+static size_t jac_sort_bytes(int NB) { return (size_t)NB * (sizeof(double) + sizeof(int)) + 16; }
 
 __global__ void __launch_bounds__(1024) k_jacobi_herm(double2* __restrict__ Aall, double2* __restrict__ Vall, int NB,
-                                                      int max_sweeps, int in_smem, double* __restrict__ w,
-                                                      int* __restrict__ sweeps) {
+                                                      int max_sweeps, int in_smem, JacPair* gpr,
+                                                      double* __restrict__ w, int* __restrict__ sweeps) {
   extern __shared__ __align__(16) unsigned char jraw[];
   const int n = NB + (NB & 1), nh = n / 2;  // even count for the round-robin (index NB is a dummy)
-  JacPair* pr2 = reinterpret_cast<JacPair*>(jraw);          // [2][nh], this step's and the previous one's
-  double* ev = reinterpret_cast<double*>(pr2 + 2 * nh);     // [NB] eigenvalues
+  // [2][nh], this step's and the previous one's
+  JacPair* pr2 = gpr ? gpr + (size_t)blockIdx.x * 2 * nh : reinterpret_cast<JacPair*>(jraw);
+  double* ev = reinterpret_cast<double*>(jraw + (gpr ? 0 : 2 * nh * sizeof(JacPair)));  // [NB] eigenvalues
   int* rank = reinterpret_cast<int*>(ev + NB);              // [NB]
   double2* mats = reinterpret_cast<double2*>(jraw + (((size_t)((unsigned char*)(rank + NB) - jraw) + 15) & ~(size_t)15));
   __shared__ double sh[64];
@@ -882,7 +886,7 @@ __global__ void __launch_bounds__(1024) k_jacobi_herm(double2* __restrict__ Aall
       const JacPair* prev = pr2 + ((step & 1) ^ 1) * nh;
       const int npw = (nh + 31) / 32;  // warps that compute rotations
       if (warp < npw && step < n - 1) {
-        for (int i = t; i < nh; i += 32 * npw) {
+        for (int i = t; i < nh; i += 32 * min(npw, nwarp)) {
           // ring position i pairs with n-1-i (i = 0: the fixed index)
           const int q0 = i == 0 ? 0 : 1 + (i + step) % (n - 1), q1 = rr_partner(q0, step, n);
           JacPair j;
@@ -981,13 +985,15 @@ __global__ void __launch_bounds__(1024) k_jacobi_herm(double2* __restrict__ Aall
 }
 
 cudaError_t launch_jacobi(const System& s, double2* A, double2* V, int max_sweeps, double* w, int* sweeps) {
-  const size_t base = jac_pair_bytes(s.NB) + 16, both = 2 * (size_t)s.NB * s.NB * sizeof(double2);
-  const int in_smem = base + both <= JAC_SMEM;
-  const size_t smem = base + (in_smem ? both : 0);
+  const size_t pairs = jac_pair_bytes(s.NB), sort = jac_sort_bytes(s.NB), both = 2 * (size_t)s.NB * s.NB * sizeof(double2);
+  const int in_smem = pairs + sort + both <= JAC_SMEM;
+  // (the split-K partials, at least nkl NB^2 values, are not in use here)
+  JacPair* gpr = pairs + sort <= JAC_SMEM ? nullptr : reinterpret_cast<JacPair*>(s.gs_part);
+  const size_t smem = (gpr ? 0 : pairs) + sort + (in_smem ? both : 0);
   const cudaError_t e = raise_smem_limit((const void*)k_jacobi_herm, smem);
   if (e != cudaSuccess) return e;
   const int nt = 32 * std::min(32, std::max(8, (s.NB + 1) / 2 + 1));  // a warp per column pair, and one for the rotations
-  k_jacobi_herm<<<s.nkl, nt, smem, s.launch_stream()>>>(A, V, s.NB, max_sweeps, in_smem, w, sweeps);
+  k_jacobi_herm<<<s.nkl, nt, smem, s.launch_stream()>>>(A, V, s.NB, max_sweeps, in_smem, gpr, w, sweeps);
   return cudaGetLastError();
 }
 

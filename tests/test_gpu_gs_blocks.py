@@ -145,3 +145,37 @@ def test_subspace_diag_sizes(cuda_lib, nb):
     assert np.abs(ov - np.eye(nb)).max() < 1e-11
     for k in range(2):
         assert rel(out[k].T @ out[k].conj(), z[k].T @ z[k].conj()) < 1e-10
+
+
+def plane_wave_bands(shape, nb, mix):
+    """Plane waves on a grid without projectors, whose H is diagonal with known values, the
+    bands b and b + nb/2 mixed by a rotation for every b in mix."""
+    from _helpers import grid_system
+    sysm = grid_system(shape, nk=1, nb=nb)
+    ln = sysm.lap_nab()
+    e, waves = [], []
+    for d, n in enumerate(shape):
+        lap = ln["lap" + "xyz"[d]]
+        m = np.arange(n)
+        e.append(-0.5 * (lap[0] + 2 * sum(lap[j] * np.cos(2 * np.pi * m * j / n) for j in range(1, 5))))
+        waves.append(np.exp(2j * np.pi * np.outer(m, np.arange(n)) / n))
+    e = (e[0][:, None, None] + e[1][:, None] + e[2]).ravel()
+    z = np.einsum("ax,by,cz->abcxyz", *waves).reshape(sysm.NL, sysm.NL)[:nb] / np.sqrt(sysm.NL * sysm.Hxyz)
+    for b in mix:
+        z[b], z[b + nb // 2] = 0.8 * z[b] + 0.6j * z[b + nb // 2], 0.6j * z[b] + 0.8 * z[b + nb // 2]
+    return sysm, z[None], np.sort(e[:nb])
+
+
+def test_subspace_diag_many_bands(cuda_lib):
+    """More than 2048 bands: more rotations in a step than a CTA has threads."""
+    from salmon_b200.rt import GpuSystem
+    nb = 2080
+    sysm, z, e = plane_wave_bands((13, 13, 13), nb, [3, 520, 1035])
+    with GpuSystem(sysm) as g:
+        g.set_vloc(np.zeros(sysm.NL))
+        g.update_projector(np.zeros((3, 1)))
+        g.gs_set_state(z)
+        esp = g.subspace_diag()
+        out = g.gs_get_state()[0]
+    assert np.abs(esp[0] - e).max() < 1e-11 * np.abs(e).max()
+    assert np.abs(out.conj() @ out.T * sysm.Hxyz - np.eye(nb)).max() < 1e-11
