@@ -12,6 +12,7 @@
 // the line.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "sgpu_internal.cuh"
@@ -155,19 +156,41 @@ static cudaError_t launch_point_t(const System& s, int mode, const PassIO& io, i
   return cudaGetLastError();
 }
 
-// The point form's time grows with the points; the march's stays at the latency of its
-// NLx steps until the CTAs fill the GPU, later the larger the plane.  Four stages with
-// the KB term, point form against march, us: complex(4) 8^3 x 256 orbitals 62 / 90, x 1024
-// 123 / 82; 20^3 x 64 131 / 123; 32^3 x 16 188 / 188; 48^3 x 4 107 / 262, x 16 279 / 246;
-// complex(8) 8^3 x 256 70 / 105, x 1024 158 / 131; 20^3 x 64 168 / 180; 32^3 x 16 237 / 423,
-// x 64 581 / 434; 48^3 x 16 427 / 583.  The lines below lie under the crossings.
-// Only with every launch choice left to the library: a KB kernel, pass form, table
-// staging, x-slab count or Taylor form set through sgpu_set_param keeps its kernels.
-bool hpsi_point_wins(const System& s, int nb, int prec) {
+// The point form's time grows with the points and, through k_uvpsi, with the points of an
+// atom; the march's stays at the latency of its NLx steps until the CTAs fill the GPU.  Both
+// therefore compare as the points of one step of the march, nb x plane.  Four stages with the
+// KB term, point form against march, us:
+//   one-row planes  complex(4) 8^3 x 128 orbitals 54 / 66, x 512 78 / 66; 20^3 x 32 95 / 119, x 64
+//                   130 / 123; 24^3 x 32 138 / 156, x 64 193 / 156; 36^3 x 16 241 / 242;
+//                   complex(8) 8^3 x 256 70 / 78, x 512 99 / 78; 12^3 x 64 71 / 90, x 128 98 / 90;
+//                   20^3 x 64 167 / 180; 24^3 x 32 168 / 230; 36^3 x 16 306 / 394, x 32 467 / 402
+//   two-row planes  (123 points an atom unless said) complex(4) 16x16x32 x 32 80 / 90, x 64 115 / 90;
+//                   32^3 x 16 115 / 131, x 32 185 / 131, with 1020 points x 4 128 / 146, x 12 172 / 148;
+//                   48^3 x 8 160 / 222, x 16 279 / 227; complex(8) 16x16x32 x 32 103 / 123, x 64
+//                   152 / 131; 32^3 x 16 158 / 189, x 32 270 / 189, with 1020 points x 8 173 / 185,
+//                   x 12 206 / 185; 48^3 x 8 238 / 284, x 12 328 / 284
+// CG's vectors (slabs > 0: the x-slabs their march would have, which shorten it; complex(8), no
+// export to S) compare by their points.  sgpu_cg, 6 bands x 4 iterations, ms, point form against
+// march: two-row planes 16x16x32 x 48 3.07 / 3.22, x 64 3.62 / 3.58; 32^3 x 12 3.01 / 3.20, x 24
+// 5.40 / 5.17, with 1020 points an atom x 1 2.25 / 2.02; 48^3 (no slabs) x 12 9.34 / 9.64, x 16 14.6 /
+// 14.1; one-row planes 24^3 with 57 points an atom x 16 2.70 / 2.83, x 32 3.28 / 3.03, with 437 points
+// x 32 3.36 / 3.42, x 48 4.91 / 4.75; 18x24x27 x 64 5.37 / 5.71.
+// The lines below lie near the crossings, where both forms take the same time to a few percent.
+// Only with every launch choice left to the library: a KB kernel, pass form, table staging,
+// x-slab count or Taylor form set through sgpu_set_param keeps its kernels.
+bool hpsi_point_wins(const System& s, int nb, int prec, int slabs) {
   if (s.kb_kernel != 0 || s.taylor_kernel != 0 || !s.pass_fixed || !s.pass_tab || s.nslab != 1) return false;
-  const long plane = (long)s.NLy * s.NLz;
-  const bool f = (prec < 0 ? s.prec : prec) == SGPU_PREC_C64;
-  return (long)nb * s.NL <= (f ? 200000 + 300 * plane : 240000 + 700 * plane);
+  const long plane = (long)s.NLy * s.NLz, mps = s.max_mps;
+  const int pr = prec < 0 ? s.prec : prec;
+  const bool f = pr == SGPU_PREC_C64, two_row = s.p2_rows[pr] > 0;
+  if (slabs > 0) {
+    long most = 240000 + 700 * plane;
+    if (slabs > 1 && two_row) most = 500000 - 480 * mps;
+    else if (slabs > 1 && s.NLz % 2 == 0) most = std::min(most, 240000 + 600 * mps);
+    return (long)nb * s.NL <= most;
+  }
+  if (two_row) return nb * plane <= (f ? std::min(18500L, 22000 - 14 * mps) : std::min(19000L, 20000 - 10 * mps));
+  return nb * plane <= (f ? 20000L : std::min(28000L, 14000 + 30 * plane));
 }
 
 // the projections of the batch must be in s.U (launch_uvpsi / launch_uvpsi_from_S)

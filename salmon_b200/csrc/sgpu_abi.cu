@@ -102,10 +102,12 @@ int one_orbital_k(const System* s, int ik) { return (ik - s->NK_s) * s->NBocc; }
 
 // One H application of a batch: projections U (gathered from io.in, or from the
 // sphere values S exported by the previous pass), the KB field W at the sphere
-// points, then the stencil pass (which may export its output to S).
-cudaError_t apply_h(System* s, int mode, sgpu::PassIO io, int o_beg, int nb, int nbk, int prec, bool u_from_S) {
+// points, then the stencil pass (which may export its output to S).  point: the
+// point-parallel form of small batches, W from the projections on the fly.
+cudaError_t apply_h(System* s, int mode, sgpu::PassIO io, int o_beg, int nb, int nbk, int prec, bool u_from_S,
+                    bool point) {
   cudaError_t e;
-  if (sgpu::hpsi_point_wins(*s, nb, prec)) {  // small batches: point-parallel, W from the projections on the fly
+  if (point) {
     if (s->nsp > 0) {
       e = u_from_S ? sgpu::launch_uvpsi_from_S(*s, s->Sbuf, o_beg, nb, nbk, true)
                    : sgpu::launch_uvpsi(*s, io.in, o_beg, nb, nbk, true, prec);
@@ -118,6 +120,9 @@ cudaError_t apply_h(System* s, int mode, sgpu::PassIO io, int o_beg, int nb, int
     io.W = s->Wbuf;
   }
   return sgpu::launch_hpsi_pass(*s, mode, io, o_beg, nb, nbk, prec);
+}
+cudaError_t apply_h(System* s, int mode, const sgpu::PassIO& io, int o_beg, int nb, int nbk, int prec, bool u_from_S) {
+  return apply_h(s, mode, io, o_beg, nb, nbk, prec, u_from_S, sgpu::hpsi_point_wins(*s, nb, prec));
 }
 
 }  // namespace
@@ -957,8 +962,10 @@ int gs_hpsi(System* s, const double2* in, double2* out, double2* tt, int nb, int
   io.out = out;
   io.tt = tt;
   const int keep = s->nslab;
-  if (s->nyblk == 1 && !sgpu::hpsi_point_wins(*s, nb, SGPU_PREC_C128)) s->nslab = std::max(1, std::min(s->nsm / std::max(1, nb), s->NLx / 8));
-  const cudaError_t e = apply_h(s, tt ? 1 : 0, io, 0, nb, nbk, SGPU_PREC_C128, false);
+  const int slabs = s->nyblk == 1 ? std::max(1, std::min(s->nsm / std::max(1, nb), s->NLx / 8)) : keep;
+  const bool point = sgpu::hpsi_point_wins(*s, nb, SGPU_PREC_C128, slabs);
+  if (!point) s->nslab = slabs;
+  const cudaError_t e = apply_h(s, tt ? 1 : 0, io, 0, nb, nbk, SGPU_PREC_C128, false, point);
   s->nslab = keep;
   CK(e);
   return 0;

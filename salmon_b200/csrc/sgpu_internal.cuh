@@ -298,8 +298,9 @@ void taylor_stage_coefs(double dt, double c[4][2]);
 cudaError_t launch_hpsi_pass(const System& s, int mode, const PassIO& io, int o_beg, int nb, int nbk, int prec = -1);
 // The same application for a small batch, one thread per point (k_point.cu), with the
 // KB term taken from the projections in s.U instead of io.W; whether that form is the
-// faster one for nb orbitals.
-bool hpsi_point_wins(const System& s, int nb, int prec = -1);
+// faster one for nb orbitals (slabs: of the ground state's vectors, the x-slabs their pass
+// would have).
+bool hpsi_point_wins(const System& s, int nb, int prec = -1, int slabs = 0);
 cudaError_t launch_hpsi_point(const System& s, int mode, const PassIO& io, int o_beg, int nb, int nbk, int prec = -1);
 int pass2_rows(int prec, int NLy, int NLz);
 // threads per CTA of the pass kernel for an NLy x NLz plane
