@@ -846,14 +846,17 @@ constexpr size_t JAC_SMEM = 220 * 1024;
 static size_t jac_pair_bytes(int NB) { return 2 * (size_t)((NB + 1) / 2) * sizeof(JacPair); }
 static size_t jac_sort_bytes(int NB) { return (size_t)NB * (sizeof(double) + sizeof(int)) + 16; }
 
+// GPR: the rotations are in gpr (a template parameter, so that the others are addressed as
+// shared memory)
+template <bool GPR>
 __global__ void __launch_bounds__(1024) k_jacobi_herm(double2* __restrict__ Aall, double2* __restrict__ Vall, int NB,
                                                       int max_sweeps, int in_smem, JacPair* gpr,
                                                       double* __restrict__ w, int* __restrict__ sweeps) {
   extern __shared__ __align__(16) unsigned char jraw[];
   const int n = NB + (NB & 1), nh = n / 2;  // even count for the round-robin (index NB is a dummy)
   // [2][nh], this step's and the previous one's
-  JacPair* pr2 = gpr ? gpr + (size_t)blockIdx.x * 2 * nh : reinterpret_cast<JacPair*>(jraw);
-  double* ev = reinterpret_cast<double*>(jraw + (gpr ? 0 : 2 * nh * sizeof(JacPair)));  // [NB] eigenvalues
+  JacPair* pr2 = GPR ? gpr + (size_t)blockIdx.x * 2 * nh : reinterpret_cast<JacPair*>(jraw);
+  double* ev = reinterpret_cast<double*>(jraw + (GPR ? 0 : 2 * nh * sizeof(JacPair)));  // [NB] eigenvalues
   int* rank = reinterpret_cast<int*>(ev + NB);              // [NB]
   double2* mats = reinterpret_cast<double2*>(jraw + (((size_t)((unsigned char*)(rank + NB) - jraw) + 15) & ~(size_t)15));
   __shared__ double sh[64];
@@ -990,10 +993,11 @@ cudaError_t launch_jacobi(const System& s, double2* A, double2* V, int max_sweep
   // (the split-K partials, at least nkl NB^2 values, are not in use here)
   JacPair* gpr = pairs + sort <= JAC_SMEM ? nullptr : reinterpret_cast<JacPair*>(s.gs_part);
   const size_t smem = (gpr ? 0 : pairs) + sort + (in_smem ? both : 0);
-  const cudaError_t e = raise_smem_limit((const void*)k_jacobi_herm, smem);
+  auto kern = gpr ? k_jacobi_herm<true> : k_jacobi_herm<false>;
+  const cudaError_t e = raise_smem_limit((const void*)kern, smem);
   if (e != cudaSuccess) return e;
   const int nt = 32 * std::min(32, std::max(8, (s.NB + 1) / 2 + 1));  // a warp per column pair, and one for the rotations
-  k_jacobi_herm<<<s.nkl, nt, smem, s.launch_stream()>>>(A, V, s.NB, max_sweeps, in_smem, gpr, w, sweeps);
+  kern<<<s.nkl, nt, smem, s.launch_stream()>>>(A, V, s.NB, max_sweeps, in_smem, gpr, w, sweeps);
   return cudaGetLastError();
 }
 
