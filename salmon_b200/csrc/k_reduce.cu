@@ -120,7 +120,9 @@ struct Nab12 {
 // one CTA per plane and 24 neighbours through L1, 20^3 x 2048 orbitals, complex(8), took
 // 1.14 ms; now 0.17 (sgpu_energy_terms: see launch_energy).  The current with this form:
 // see current_stencil.
-// out[o][block][4] = {sum |e|^2, F/2, G/2, H/2}, or [o][block][2] = {Re tpsum, 0}.
+// Few orbitals leave SMs idle behind a chain of NLx steps: the march is then cut into slabs
+// of SX planes, one CTA each (see march_slabs).
+// out[o][block][slab][4] = {sum |e|^2, F/2, G/2, H/2}, or [o][block][slab][2] = {Re tpsum, 0}.
 struct FwdCoef {
   double lap0_2;    // EKIN: -(lapx(0)+lapy(0)+lapz(0))/2
   double lap[12];   // EKIN: lapx(1:4), lapy(1:4), lapz(1:4)
@@ -129,7 +131,7 @@ struct FwdCoef {
 
 template <typename R, bool EKIN>
 __global__ void __launch_bounds__(256, 2) k_fwd_march(const C2<R>* __restrict__ zu, int NLx, int NLy, int NLz, int GB,
-                                                      int nblk, int NBocc, const double* __restrict__ kAc,
+                                                      int nblk, int SX, int NBocc, const double* __restrict__ kAc,
                                                       const FwdCoef c, double* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double sh[32 * 4];
@@ -137,6 +139,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_march(const C2<R>* __restrict__ 
   const int RB = (GB + 4) * NLz;
   const int o = blockIdx.x / nblk, h = blockIdx.x - o * nblk, t = threadIdx.x, nt = blockDim.x;
   const int NYZ = NLy * NLz, rows = min(GB, NLy - h * GB);
+  const int x_beg = blockIdx.y * SX, x_end = min(x_beg + SX, NLx);  // (never empty)
   const C2<R>* E = zu + (size_t)o * NLx * NYZ;
   const int y0 = 2 * (t / NLz), z = t - (t / NLz) * NLz;
   const bool act = y0 < rows, two = y0 + 1 < rows;
@@ -158,19 +161,19 @@ __global__ void __launch_bounds__(256, 2) k_fwd_march(const C2<R>* __restrict__ 
   auto load = [&](int x, int i, bool ok) -> double2 {
     return ok ? to_d2(__ldg(E + (size_t)x * NYZ + i)) : make_double2(0, 0);
   };
-  // register queues: at phase P (plane x = 5i + P) plane x+m sits in slot (P+m) % 5
+  // register queues: at phase P (plane x = x_beg + 5i + P) plane x+m sits in slot (P+m) % 5
   double2 qa[5], qb[5];
 #pragma unroll
   for (int m = 0; m < 5; ++m) {
-    const int xm = m % NLx;
+    const int xm = (x_beg + m) % NLx;
     qa[m] = load(xm, own, act);
     qb[m] = load(xm, own_b, two);
   }
-  int xn = 5 % NLx;
+  int xn = (x_beg + 5) % NLx;
   C2<R> na = __ldg(E + (size_t)xn * NYZ + own), nb = __ldg(E + (size_t)xn * NYZ + own_b);  // in flight
   xn = xn + 1 < NLx ? xn + 1 : 0;
   double v[4] = {0, 0, 0, 0};
-  int x = 0;
+  int x = x_beg;
   auto step = [&](auto phase) -> bool {
     constexpr int P = decltype(phase)::value;
     double2* pl = buf + (x & 1) * RB;
@@ -236,7 +239,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_march(const C2<R>* __restrict__ 
     nb = __ldg(E + (size_t)xn * NYZ + own_b);
     xn = xn + 1 < NLx ? xn + 1 : 0;
     ++x;
-    return x < NLx;
+    return x < x_end;
   };
   for (;;) {
     if (!step(std::integral_constant<int, 0>{})) break;
@@ -247,12 +250,13 @@ __global__ void __launch_bounds__(256, 2) k_fwd_march(const C2<R>* __restrict__ 
   }
   block_sum<4>(v, sh);
   if (t == 0) {
+    const size_t row = (size_t)blockIdx.x * gridDim.y + blockIdx.y;
     if (EKIN) {
-      out[2 * (size_t)blockIdx.x] = c.lap0_2 * v[0] - v[1] + 2.0 * v[2];
-      out[2 * (size_t)blockIdx.x + 1] = 0.0;
+      out[2 * row] = c.lap0_2 * v[0] - v[1] + 2.0 * v[2];
+      out[2 * row + 1] = 0.0;
     } else {
 #pragma unroll
-      for (int m = 0; m < 4; ++m) out[4 * (size_t)blockIdx.x + m] = v[m];
+      for (int m = 0; m < 4; ++m) out[4 * row + m] = v[m];
     }
   }
 }
@@ -263,10 +267,20 @@ int march_rows(int NLy, int NLz) {
   const int most = std::max(2, 2 * (256 / NLz)), nblk = (NLy + most - 1) / most;
   return ((NLy + nblk - 1) / nblk + 1) / 2 * 2;
 }
-int march_blocks(int NLy, int NLz) {
+static int march_blocks(int NLy, int NLz) {
   const int GB = march_rows(NLy, NLz);
   return (NLy + GB - 1) / GB;
 }
+// slabs of the march: as many as two CTAs per SM take, each of at least four planes (a slab
+// reads five planes before its first step).
+// Without slabs and with them, complex(4), us: sgpu_energy_terms 18x24x27 x 16 orbitals 64 / 55,
+// 40^3 x 1 107 / 80, x 64 123 / 119; sgpu_current 36^3 x 4 90 / 66.
+static int march_slabs(const System& s) {
+  const int ctas = s.norb * march_blocks(s.NLy, s.NLz);
+  const int most = std::max(1, std::min(2 * s.nsm / ctas, s.NLx / 4)), SX = (s.NLx + most - 1) / most;
+  return (s.NLx + SX - 1) / SX;
+}
+int march_parts(const System& s) { return march_blocks(s.NLy, s.NLz) * march_slabs(s); }
 
 template <typename R, bool EKIN>
 static cudaError_t fwd_march(System& s, double* out, int& nx) {
@@ -278,13 +292,14 @@ static cudaError_t fwd_march(System& s, double* out, int& nx) {
       c.nab[4 * d + n] = s.nab[d][n + 1];
     }
   const int GB = march_rows(s.NLy, s.NLz);
-  nx = march_blocks(s.NLy, s.NLz);
+  const int nblk = march_blocks(s.NLy, s.NLz), nslab = march_slabs(s);
+  nx = nblk * nslab;
   const int nt = (GB / 2 * s.NLz + 31) / 32 * 32;
   const size_t smem = 2 * (size_t)(GB + 4) * s.NLz * sizeof(double2);
   const cudaError_t e = raise_smem_limit((const void*)k_fwd_march<R, EKIN>, smem);
   if (e != cudaSuccess) return e;
-  k_fwd_march<R, EKIN><<<s.norb * nx, nt, smem, s.launch_stream()>>>((const C2<R>*)s.zu, s.NLx, s.NLy, s.NLz, GB, nx,
-                                                                     s.NBocc, s.kAc_d, c, out);
+  k_fwd_march<R, EKIN><<<dim3(s.norb * nblk, nslab), nt, smem, s.launch_stream()>>>(
+      (const C2<R>*)s.zu, s.NLx, s.NLy, s.NLz, GB, nblk, (s.NLx + nslab - 1) / nslab, s.NBocc, s.kAc_d, c, out);
   return cudaGetLastError();
 }
 

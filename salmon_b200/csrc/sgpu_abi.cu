@@ -527,7 +527,7 @@ int sgpu_create(const sgpu_desc* d, int precision, sgpu_handle* out) {
   if ((e = dalloc(&s->vloc64, s->NL)) != cudaSuccess) return bail(cuda_fail(e, "alloc vloc64"));
   if ((e = dalloc(&s->vloc32, s->NL)) != cudaSuccess) return bail(cuda_fail(e, "alloc vloc32"));
   const size_t nchunk = (s->norb + 63) / 64;
-  s->part_rows = std::max(6, sgpu::march_blocks(s->NLy, s->NLz));  // (the fixed shapes use up to 6)
+  s->part_rows = std::max(6, sgpu::march_parts(*s));  // (the fixed shapes use up to 6)
   s->red_elems = std::max<size_t>({nchunk * s->NL, 4 * (size_t)s->norb + 64, (size_t)s->NL + 64,
                                    sgpu::current_red_elems(s->norb, s->part_rows)});
   if ((size_t)((s->NL + 255) / 256) * nchunk < 2 * (size_t)s->nsm)  // small grids: the density in chunks of 16 orbitals

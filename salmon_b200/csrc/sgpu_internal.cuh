@@ -344,8 +344,8 @@ cudaError_t launch_current(System& s, double* jav_dev);
 cudaError_t launch_current_proj(System& s);
 // reduction scratch (doubles) that launch_current and launch_energy need
 size_t current_red_elems(int norb, int rows);
-// row blocks of the generic current / energy march (parts per orbital)
-int march_blocks(int NLy, int NLz);
+// CTAs of the any-shape current / energy march per orbital (its partial sums)
+int march_parts(const System& s);
 // per-orbital kinetic and nonlocal energies summed (device, 2 doubles)
 cudaError_t launch_energy(System& s, double* e_dev);
 

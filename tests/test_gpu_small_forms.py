@@ -82,6 +82,24 @@ def test_current_and_energy_march(cuda_lib, precision, shape):
 
 
 @pytest.mark.parametrize("precision", ["c128", "c64"])
+@pytest.mark.parametrize("shape,nb", [((22, 9, 11), 1), ((13, 34, 16), 3), ((10, 8, 8), 80), ((31, 36, 30), 2)])
+def test_march_slabs(cuda_lib, precision, shape, nb):
+    """Few orbitals: the march in slabs of at least four planes, the last one shorter."""
+    from salmon_b200.rt import GpuSystem
+    sysm, kAc, vloc, zu = S.small_system(*shape, nk=1, nb=nb, seed=5)
+    z = zu if precision == "c128" else zu.astype(np.complex64).astype(np.complex128)
+    with GpuSystem(sysm, precision) as g:
+        g.set_state(zu)
+        g.set_vloc(vloc)
+        assert rel(g.current_RT(kAc), O.current(sysm, kAc, z)) < 1e-11
+        assert rel(g.energy_terms(kAc), O.energy_terms(sysm, kAc, z)) < 1e-11
+        g.update_projector(kAc)
+        g.hamiltonian(0.004, flag_current=True)
+        z1 = np.asarray(g.get_state(), np.complex128)
+        assert rel(g.current_RT(kAc), O.current(sysm, kAc, z1)) < 1e-11
+
+
+@pytest.mark.parametrize("precision", ["c128", "c64"])
 @pytest.mark.parametrize("cur_fixed", [1, 2])
 @pytest.mark.parametrize("shape", [(1, 32, 32), (3, 32, 32), (4, 48, 48), (5, 32, 32), (6, 48, 48)])
 def test_current_of_few_planes(cuda_lib, precision, cur_fixed, shape):
