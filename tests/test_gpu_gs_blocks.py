@@ -132,6 +132,60 @@ def test_cg_projections(cuda_lib, grid, nk, nb, orthonormal):
     assert rel(esp, esp_ref) < 1e-9
 
 
+def tpa_cg(sysm, kAc, vloc, z, ncg):
+    """CG with the Teter-Payne-Allan factor as it is defined, projection by projection."""
+    from oracle import net_oracle as N
+    d = sysm.desc()
+    lap3, nab3 = (np.array([list(getattr(d, p + c)) for c in "xyz"]) for p in ("lap", "nab"))
+    shape, w = (sysm.NLx, sysm.NLy, sysm.NLz), sysm.Hxyz
+    _, zproj = O.update_projector(sysm, kAc)
+    z = z.copy()
+    for k in range(sysm.nk_local):
+        H = lambda x: O.hpsi(sysm, kAc, vloc, zproj, k + 1, x, want_tt=True)  # noqa: E731
+        dot = lambda a, b: np.vdot(a, b) * w  # noqa: E731
+
+        def project(x, lower):
+            for u in lower:
+                x = x - u * dot(u, x)
+            return x
+
+        for b in range(sysm.NB):
+            x, lower = z[k, b], z[k, :b]
+            for u in lower:
+                x = x - u * dot(u, x).real
+            x = x / np.sqrt(dot(x, x).real)
+            hx, tx = H(x)
+            for it in range(ncg):
+                e, t = dot(x, hx).real, dot(x, tx).real
+                g = project(hx - e * x, lower)
+                h = project(N.tpa_apply(g, shape, kAc[:, k], max(t, 1e-6), lap3, nab3), lower)
+                h = h - x * dot(x, h)
+                s = dot(g, h).real
+                p = h if it == 0 else h + s / s_old * p
+                s_old = s
+                q = p - x * dot(x, p)
+                q = q / np.sqrt(dot(q, q).real)
+                hq, tq = H(q)
+                c, f = dot(x, hq), dot(q, hq).real
+                ev = 0.5 * (e + f - np.sqrt((e - f) ** 2 + 4 * abs(c) ** 2))
+                cx = c / (ev - e)
+                cp = 1 / np.sqrt(1 + abs(cx) ** 2)
+                x, hx, tx = (cp * (cx * a + y) for a, y in ((x, q), (hx, hq), (tx, tq)))
+            z[k, b] = x / np.sqrt(dot(x, x).real)
+    return z
+
+
+@pytest.mark.parametrize("grid,nk,nb", [((8, 9, 12), 2, 9), ((16, 16, 16), 1, 128)])  # clusters, the whole GPU
+def test_cg_projections_preconditioned(cuda_lib, grid, nk, nb):
+    sysm, kAc, vloc, z = raw_system(grid, nk, nb)
+    z = S.orthonormalise(z, sysm.Hxyz)
+    with handle(sysm, kAc, vloc, z) as g:
+        g.set_cg_preconditioner("tpa")
+        g.cg(3)
+        out = g.gs_get_state()
+    assert rel(out, tpa_cg(sysm, kAc, vloc, z, 3)) < 1e-9
+
+
 @pytest.mark.parametrize("nb", [7, 82, 84, 128])  # A and V in shared memory up to 82 bands
 def test_subspace_diag_sizes(cuda_lib, nb):
     sysm, kAc, vloc, z = raw_system((8, 9, 10), 2, nb)
