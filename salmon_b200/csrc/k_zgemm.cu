@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(128) k_zgemm_nn(const double2* X, size_t xstri
                                                  size_t zstride, int ldz, int M, int N, int NL, const double2* base,
                                                  double2* out, size_t ostride, const int* __restrict__ skip) {
   __shared__ double2 sx[ZST2][ZK][ZP], sz[ZST2][ZT][ZROW];
-  const int k = blockIdx.z, n0 = blockIdx.y * ZT, p0 = blockIdx.x * ZP;
+  const int npt = (NL + ZP - 1) / ZP, k = blockIdx.x / npt, n0 = blockIdx.y * ZT, p0 = (blockIdx.x - k * npt) * ZP;
   if (skip && skip[k]) return;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const double2* Xk = X + k * xstride;
@@ -218,7 +218,8 @@ static cudaError_t launch_hn(const System& s, const double2* A, int M, const dou
 static cudaError_t launch_nn(const System& s, const double2* X, int M, const double2* Z, size_t zstride, int ldz, int N,
                              const double2* base, double2* out, const int* skip = nullptr) {
   const size_t ks = (size_t)s.NB * s.NL;
-  k_zgemm_nn<<<dim3((s.NL + ZP - 1) / ZP, (N + ZT - 1) / ZT, s.nkl), 128, 0, s.launch_stream()>>>(
+  // (k-points in the first grid dimension: the others end at 65535)
+  k_zgemm_nn<<<dim3(s.nkl * ((s.NL + ZP - 1) / ZP), (N + ZT - 1) / ZT), 128, 0, s.launch_stream()>>>(
       X, ks, Z, zstride, ldz, M, N, s.NL, base, out, ks, skip);
   return cudaGetLastError();
 }

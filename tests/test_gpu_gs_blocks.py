@@ -132,6 +132,20 @@ def test_cg_projections(cuda_lib, grid, nk, nb, orthonormal):
     assert rel(esp, esp_ref) < 1e-9
 
 
+def test_gram_schmidt_many_k_points(cuda_lib):
+    """More k-points than the second and third dimension of a grid can count."""
+    from _helpers import grid_system
+    from salmon_b200.rt import GpuSystem
+    sysm = grid_system((3, 3, 3), nk=65600, nb=3)
+    rng = np.random.default_rng(8)
+    z = rng.standard_normal((65600, 3, sysm.NL)) + 1j * rng.standard_normal((65600, 3, sysm.NL))
+    with GpuSystem(sysm) as g:
+        g.gs_set_state(z)
+        g.gram_schmidt()
+        out = g.gs_get_state()
+    assert rel(out, O.gram_schmidt(sysm, z)) < 1e-12
+
+
 def tpa_cg(sysm, kAc, vloc, z, ncg):
     """CG with the Teter-Payne-Allan factor as it is defined, projection by projection."""
     from oracle import net_oracle as N
