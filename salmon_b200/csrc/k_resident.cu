@@ -552,15 +552,25 @@ bool resident_step_fits(const System& s) {
   return res_dispatch(s, [](auto, auto, auto, auto, auto) {});
 }
 
-// The resident form is the default (SGPU_PARAM_TAYLOR_KERNEL 0) where it measured
-// faster than the stencil passes: 16x16 planes (16^3 grid x 64 k x 16 bands:
-// complex(4) 0.181 against 0.201 ms per step, complex(8) 0.326 against 0.437 ms).
+// The resident form is the default (SGPU_PARAM_TAYLOR_KERNEL 0) where it is not slower than
+// the stencil passes: on 16x16 planes, up to a number of waves of its CTAs (one per SM), whose
+// time grows by whole waves.  Potential update, step and current, us, resident / passes:
+// complex(4) 16^3 (four orbitals a CTA) x 512 orbitals 223 / 243, x 608 331 / 286, x 1024 338 / 335, x 2048
+// 571 / 538; 32x16x16 (two) x 256 245 / 252, x 512 381 / 340; complex(8) 16^3 (two) x 256 201 / 258, x 1024
+// 498 / 530, x 2048 810 / 830, x 2560 1007 / 994; 24x16x16 (one) x 512 450 / 477, x 608 546 / 521.
 // Elsewhere it is slower (20^3 x 2048 orbitals: complex(4) 1.27 against 0.73 ms,
 // complex(8) 1.95 against 1.47 ms): with one CTA per SM the latency of the
 // projector-table loads in each stage's KB phase is not hidden behind other CTAs'
 // work, and the 20x20 forms spill.  The step tuner measures both per shape.
 bool resident_step_default(const System& s) {
-  return s.NLy == 16 && s.NLz == 16 && resident_step_fits(s);
+  if (s.NLy != 16 || s.NLz != 16) return false;
+  int groups = 0, waves = 0;
+  res_dispatch(s, [&](auto tag, auto, auto, auto nbc, auto) {
+    constexpr int NBC = decltype(nbc)::value;
+    groups = s.nkl * ((s.NBocc + NBC - 1) / NBC);
+    waves = std::is_same<decltype(tag), float>::value ? 1 : (NBC == 2 ? 7 : 4);
+  });
+  return groups > 0 && groups <= waves * s.nsm;
 }
 
 cudaError_t launch_taylor_resident(const System& s, void* zu, double dt, double* cur, void* S) {
