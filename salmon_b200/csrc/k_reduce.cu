@@ -129,7 +129,7 @@ struct FwdCoef {
   double nab[12];   // nabx(1:4), naby(1:4), nabz(1:4)
 };
 
-template <typename R, bool EKIN>
+template <typename R, bool EKIN, bool SLABS>
 __global__ void __launch_bounds__(256, 2) k_fwd_march(const C2<R>* __restrict__ zu, int NLx, int NLy, int NLz, int GB,
                                                       int nblk, int SX, int NBocc, const double* __restrict__ kAc,
                                                       const FwdCoef c, double* __restrict__ out) {
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_march(const C2<R>* __restrict__ 
   const int RB = (GB + 4) * NLz;
   const int o = blockIdx.x / nblk, h = blockIdx.x - o * nblk, t = threadIdx.x, nt = blockDim.x;
   const int NYZ = NLy * NLz, rows = min(GB, NLy - h * GB);
-  const int x_beg = blockIdx.y * SX, x_end = min(x_beg + SX, NLx);  // (never empty)
+  const int x_beg = SLABS ? blockIdx.y * SX : 0, x_end = SLABS ? min(x_beg + SX, NLx) : NLx;  // (never empty)
   const C2<R>* E = zu + (size_t)o * NLx * NYZ;
   const int y0 = 2 * (t / NLz), z = t - (t / NLz) * NLz;
   const bool act = y0 < rows, two = y0 + 1 < rows;
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_march(const C2<R>* __restrict__ 
   C2<R> na = __ldg(E + (size_t)xn * NYZ + own), nb = __ldg(E + (size_t)xn * NYZ + own_b);  // in flight
   xn = xn + 1 < NLx ? xn + 1 : 0;
   double v[4] = {0, 0, 0, 0};
-  int x = x_beg;
+  int x = x_beg, left = x_end - x_beg;
   auto step = [&](auto phase) -> bool {
     constexpr int P = decltype(phase)::value;
     double2* pl = buf + (x & 1) * RB;
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_march(const C2<R>* __restrict__ 
     nb = __ldg(E + (size_t)xn * NYZ + own_b);
     xn = xn + 1 < NLx ? xn + 1 : 0;
     ++x;
-    return x < x_end;
+    return --left > 0;
   };
   for (;;) {
     if (!step(std::integral_constant<int, 0>{})) break;
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(256, 2) k_fwd_march(const C2<R>* __restrict__ 
   }
   block_sum<4>(v, sh);
   if (t == 0) {
-    const size_t row = (size_t)blockIdx.x * gridDim.y + blockIdx.y;
+    const size_t row = SLABS ? (size_t)blockIdx.x * gridDim.y + blockIdx.y : blockIdx.x;
     if (EKIN) {
       out[2 * row] = c.lap0_2 * v[0] - v[1] + 2.0 * v[2];
       out[2 * row + 1] = 0.0;
@@ -271,16 +271,20 @@ static int march_blocks(int NLy, int NLz) {
   const int GB = march_rows(NLy, NLz);
   return (NLy + GB - 1) / GB;
 }
-// slabs of the march: as many as two CTAs per SM take, each of at least four planes (a slab
-// reads five planes before its first step).
+// Slabs of the march, each of at least four planes (a slab reads five planes before its first
+// step): as many as two CTAs per SM take for the energy, one for the current, which runs
+// beside a step's density and potential: two delay those (step at 24x8x48, complex(8), 98
+// orbitals 283 us without slabs, 282 with one, 289 with two).
 // Without slabs and with them, complex(4), us: sgpu_energy_terms 18x24x27 x 16 orbitals 64 / 55,
 // 40^3 x 1 107 / 80, x 64 123 / 119; sgpu_current 36^3 x 4 90 / 66.
-static int march_slabs(const System& s) {
+static int march_slabs(const System& s, int ctas_per_sm) {
   const int ctas = s.norb * march_blocks(s.NLy, s.NLz);
-  const int most = std::max(1, std::min(2 * s.nsm / ctas, s.NLx / 4)), SX = (s.NLx + most - 1) / most;
+  const int most = std::max(1, std::min(ctas_per_sm * s.nsm / ctas, s.NLx / 4)), SX = (s.NLx + most - 1) / most;
   return (s.NLx + SX - 1) / SX;
 }
-int march_parts(const System& s) { return march_blocks(s.NLy, s.NLz) * march_slabs(s); }
+int march_parts(const System& s) {
+  return march_blocks(s.NLy, s.NLz) * std::max(march_slabs(s, 1), march_slabs(s, 2));
+}
 
 template <typename R, bool EKIN>
 static cudaError_t fwd_march(System& s, double* out, int& nx) {
@@ -292,13 +296,15 @@ static cudaError_t fwd_march(System& s, double* out, int& nx) {
       c.nab[4 * d + n] = s.nab[d][n + 1];
     }
   const int GB = march_rows(s.NLy, s.NLz);
-  const int nblk = march_blocks(s.NLy, s.NLz), nslab = march_slabs(s);
+  const int nblk = march_blocks(s.NLy, s.NLz), nslab = march_slabs(s, EKIN ? 2 : 1);
   nx = nblk * nslab;
   const int nt = (GB / 2 * s.NLz + 31) / 32 * 32;
   const size_t smem = 2 * (size_t)(GB + 4) * s.NLz * sizeof(double2);
-  const cudaError_t e = raise_smem_limit((const void*)k_fwd_march<R, EKIN>, smem);
+  // (bounds known at compile time without slabs: 172.5 against 173.4 us at 20^3 x 2048)
+  auto kern = nslab > 1 ? k_fwd_march<R, EKIN, true> : k_fwd_march<R, EKIN, false>;
+  const cudaError_t e = raise_smem_limit((const void*)kern, smem);
   if (e != cudaSuccess) return e;
-  k_fwd_march<R, EKIN><<<dim3(s.norb * nblk, nslab), nt, smem, s.launch_stream()>>>(
+  kern<<<dim3(s.norb * nblk, nslab), nt, smem, s.launch_stream()>>>(
       (const C2<R>*)s.zu, s.NLx, s.NLy, s.NLz, GB, nblk, (s.NLx + nslab - 1) / nslab, s.NBocc, s.kAc_d, c, out);
   return cudaGetLastError();
 }
