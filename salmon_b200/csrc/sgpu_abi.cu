@@ -1064,13 +1064,14 @@ int sgpu_cg(sgpu_handle h, int ncg, double* esp_var, int* iters) {
 int sgpu_set_vpsl(sgpu_handle h, const double* vpsl) {
   if (!valid(h) || !vpsl) return fail(SGPU_ERR_ARG, "sgpu_set_vpsl: null argument");
   System* s = h;
-  if (!s->vpsl) {
-    CK(cudaMalloc(&s->vpsl, (size_t)s->NL * sizeof(double)));
-    CK(cudaMalloc(&s->rho_d, (size_t)s->NL * sizeof(double)));
-    CK(cudaMalloc(&s->exc_d, (2 + 2 * sgpu::XC_PARTS + 1) * sizeof(double)));  // energies, partial energies, counter
+  if (!s->vpsl) {  // (allocated last: it stands for all of them)
+    if (!s->rho_d) CK(cudaMalloc(&s->rho_d, (size_t)s->NL * sizeof(double)));
+    if (!s->exc_d)  // energies, partial energies, counter
+      CK(cudaMalloc(&s->exc_d, (2 + 2 * sgpu::XC_PARTS + 1) * sizeof(double)));
     s->xc_part = s->exc_d + 2;
     s->xc_count = (unsigned*)(s->xc_part + 2 * sgpu::XC_PARTS);
     CK(cudaMemsetAsync(s->xc_count, 0, sizeof(unsigned), s->stream));
+    CK(cudaMalloc(&s->vpsl, (size_t)s->NL * sizeof(double)));
   }
   CK(cudaMemcpyAsync(s->vpsl, vpsl, (size_t)s->NL * sizeof(double), cudaMemcpyHostToDevice, s->stream));
   CK(cudaStreamSynchronize(s->stream));
