@@ -38,7 +38,7 @@ DT = 0.08
 # ncu dram__bytes_read.sum + dram__bytes_write.sum of one Taylor-stage launch, per
 # orbital, from the capture in profiles/k_hpsi_pass2_c64_c128.md (512 orbitals;
 # traffic grows with the orbital count).
-NCU_TRAFFIC_BYTES_PER_ORBITAL = {("taylor_stage", "c64", 32): 337.961472e6 / 512}
+NCU_TRAFFIC_BYTES_PER_ORBITAL = {("taylor_stage", "c64", 32): 341.046528e6 / 512}
 
 
 def parse():

@@ -346,7 +346,8 @@ enum {
   SGPU_PARAM_TAYLOR_KERNEL = 8, /* Taylor step: 1 four stencil passes over all orbitals (any grid), 2
                                  the orbitals of a band group resident in one CTA's shared memory for
                                  the whole step (16x16, 16x32 and 20x20 planes where they fit), 0 the
-                                 resident form where it is the faster one (16x16 planes), else the
+                                 resident form where it is not slower (16x16 planes, up to one wave
+                                 of its CTAs in complex(4), four to seven in complex(8)), else the
                                  passes                                                              */
   SGPU_PARAM_NSP = 9,         /* sphere points of the handle (read only): the union of the
                                  projectors' points, a key of the launch-shape table              */
@@ -368,13 +369,16 @@ enum { SGPU_CG_PLAIN = 0, SGPU_CG_TPA = 1, SGPU_CG_LEARNED = 2 };
 int sgpu_set_param(sgpu_handle h, int param, int value);
 int sgpu_get_param(sgpu_handle h, int param, int* value);
 
-/* Autotuner: times `reps` H applications of the resident orbitals (projections,
- * KB field, stencil pass) for every launch shape it knows (x-slabs per orbital
- * 1, 2, 4; KB term by the band-group tile kernel, returned as split 0, or by
- * the band-quad kernel with projection split 1, 2, 4, 8), keeps the fastest in
- * the handle (SGPU_PARAM_NSLAB, SGPU_PARAM_KB_KERNEL, SGPU_PARAM_UVPSI_SPLIT)
- * and returns it (any output pointer may be NULL).  The resident orbitals are not
- * modified.  No reference counterpart; the nearest is auto_blocking
+/* Autotuner of the H application's explicit shapes: times `reps` H applications
+ * of the resident orbitals (projections, KB field, stencil pass) for x-slabs per
+ * orbital 1, 2, 4 and the KB term by the band-group tile kernel, returned as
+ * split 0, or by the band-quad kernel with projection split 1, 2, 4, 8; keeps
+ * the fastest of these in the handle (SGPU_PARAM_NSLAB, SGPU_PARAM_KB_KERNEL,
+ * SGPU_PARAM_UVPSI_SPLIT) and returns it (any output pointer may be NULL).  What
+ * the library chooses by itself (the point-parallel form of small batches, atoms
+ * of few points staged whole) is not among them and can be faster: it is off as
+ * long as a KB kernel is set, and sgpu_autotune_step compares with it.  The
+ * resident orbitals are not modified.  No reference counterpart; the nearest is auto_blocking
  * (modules/opt_variables.f90:340-353). */
 int sgpu_autotune(sgpu_handle h, int reps, int* nslab, int* split, double* ms_per_apply);
 

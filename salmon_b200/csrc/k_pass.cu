@@ -418,8 +418,9 @@ __global__ void __launch_bounds__(512) k_hpsi_pass(const PassArgs<R> a) {
 // The x terms are added first, and the sum starts at the centre term (see m2A).  One second
 // derivative accumulator per point: a second one for y, as in k_hpsi_pass, spills at three
 // CTAs per SM (0.412 against 0.377 ms at 32^3).  Complex(8) adds the small terms first and
-// starts the first derivatives by a product, complex(4) neither: whichever left no spill
-// there.  KB: W and S are both given (a Taylor stage).  Measured times: see pass2_rows.
+// starts the first derivatives by a product, complex(4) neither: whichever spilled least (no
+// complex(4) instance spills; ten of the sixteen complex(8) ones do, 4 to 24 bytes, of the
+// Taylor stages with KB the 16x16 one).  KB: W and S are both given (a Taylor stage).  Measured times: see pass2_rows.
 constexpr int P2_NS = 3;  // planes in shared memory = phases of the unrolled march
 
 template <typename R> struct P2Geom { static constexpr int RZ = std::is_same<R, float>::value ? 2 : 1; };

@@ -118,8 +118,12 @@ struct Nab12 {
 // so tpsum = sum conj(e) (lap0_2 e - 0.5 v - i w) (stencil/F90/total_energy.f90:93-180) needs
 // the forward neighbours only: half of the arithmetic and of the shared-memory reads.  With
 // one CTA per plane and 24 neighbours through L1, 20^3 x 2048 orbitals, complex(8), took
-// 1.14 ms; now 0.17 (sgpu_energy_terms: see launch_energy).  The current with this form:
-// see current_stencil.
+// 1.14 ms; now 0.17 (sgpu_energy_terms: see launch_energy).  The norm, Laplacian and k parts are
+// summed over the block and subtracted at the end, so the large terms cancel in the sums and
+// not point by point; the rounding is the same, that of the products.  Restated on the host
+// against extended precision, 20^3: a smooth orbital 7.0e-15 (point by point 8.6e-15), one
+// that is constant to 1e-2 1.5e-11 (2.6e-11), to 1e-4 3.0e-7 (2.5e-7).  The current with this
+// form: see current_stencil.
 // Few orbitals leave SMs idle behind a chain of NLx steps: the march is then cut into slabs
 // of SX planes, one CTA each (see march_slabs).
 // out[o][block][slab][4] = {sum |e|^2, F/2, G/2, H/2}, or [o][block][slab][2] = {Re tpsum, 0}.

@@ -160,8 +160,9 @@ class GpuSystem:
         return v.value
 
     def autotune(self, reps: int = 5):
-        """Times every launch shape the library knows on the resident orbitals and
-        keeps the fastest; returns (nslab, uvpsi_split, ms per H application)."""
+        """Times the explicit launch shapes of the H application (x-slabs, tile or band-quad
+        KB kernel) on the resident orbitals and keeps the fastest of them; returns (nslab,
+        uvpsi_split, ms per H application).  autotune_step also tries the library's own choice."""
         ns, sp, ms = C.c_int(), C.c_int(), C.c_double()
         call("sgpu_autotune", self._h, int(reps), C.byref(ns), C.byref(sp), C.byref(ms))
         return ns.value, sp.value, ms.value
